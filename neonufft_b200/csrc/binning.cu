@@ -66,6 +66,7 @@ constexpr int kBinUnroll = 4;
 template <int DIM>
 __device__ __forceinline__ i64 tile_linear_d(const BinGeom& g, const i64 (&t)[3]) {
   if (DIM == 3 && g.zmajor) return t[2] + i64(g.ntiles[2]) * (t[0] + i64(g.ntiles[0]) * t[1]);
+  if (DIM == 2 && g.strip) return t[1] + i64(g.ntiles[1]) * t[0];
   i64 lin = 0, mul = 1;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
@@ -178,6 +179,10 @@ __global__ void __launch_bounds__(kBinBlock)
       r[u].frac[0] = T(fr[0]);
       r[u].frac[1] = T(fr[1]);
       r[u].frac[2] = T(fr[2]);
+      if (DIM < 3 && g.strip) {
+        r[u].local = u32(i0[0]);
+        if (DIM == 2) set_strip_row(r[u], i0[1]);
+      }
     }
     u32 pos[kBinUnroll];
 #pragma unroll

@@ -146,11 +146,13 @@ struct BinGeom {
   double offset[3];   // affine pre-transform (type 3); 0 / 1 otherwise
   double scale[3];
   int zmajor;         // 3D: bins ordered plane-fastest, tz + ntz (tx + ntx ty); else x-fastest
+  int strip;          // 1D, 2D: bins ordered row-fastest, ty + nty tx, records with absolute cells
 };
 
 // Linear bin index of tile coordinates t[0..dim).
 __host__ __device__ __forceinline__ i64 tile_linear(const BinGeom& g, const i64* t) {
   if (g.dim == 3 && g.zmajor) return t[2] + i64(g.ntiles[2]) * (t[0] + i64(g.ntiles[0]) * t[1]);
+  if (g.dim == 2 && g.strip) return t[1] + i64(g.ntiles[1]) * t[0];
   i64 lin = 0, mul = 1;
   for (int d = 0; d < g.dim; ++d) {
     lin += t[d] * mul;
@@ -193,6 +195,26 @@ struct alignas(16) PointRec {
 };
 static_assert(sizeof(PointRec<float>) == 32 && sizeof(PointRec<double>) == 32,
               "point records are one 32-byte sector");
+
+// Strip-ordered 1D and 2D point sets (BinGeom::strip) store the absolute first cell: x in `local`
+// and, in 2D, the first row in the bits of the unused third fraction.
+__device__ __forceinline__ void set_strip_row(PointRec<float>& r, int y) {
+  r.frac[2] = __int_as_float(y);
+}
+__device__ __forceinline__ void set_strip_row(PointRec<double>& r, int y) {
+  r.frac[2] = __longlong_as_double(static_cast<long long>(y));
+}
+__device__ __forceinline__ int strip_row(const PointRec<float>& r) {
+  return __float_as_int(r.frac[2]);
+}
+__device__ __forceinline__ int strip_row(const PointRec<double>& r) {
+  return int(__double_as_longlong(r.frac[2]));
+}
+// Cells per strip: 8 (fewer rows flushed per point than 4), 4 where a row of the window would
+// take more than 64 registers.
+__host__ __device__ constexpr int strip_width(size_t real_bytes, int w) {
+  return real_bytes == 8 && w > 8 ? 4 : 8;
+}
 
 // The whole sector of a record, as two 16-byte vectors (copies keep the sector whole).
 template <typename T>

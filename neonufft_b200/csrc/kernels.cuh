@@ -89,6 +89,9 @@ template <typename T>
 void launch_spread(const SpreadArgs<T>& a, cudaStream_t stream);
 template <typename T>
 void launch_spread_zwin(const SpreadArgs<T>& a, cudaStream_t stream);
+// 1D and 2D spreading of strip-ordered points (strip.cu).
+template <typename T>
+void launch_spread_strip(const SpreadArgs<T>& a, cudaStream_t stream);
 // Method 5: 3D single-precision spreading on the tcgen05 tensor cores (spread_tc.cu).
 void launch_spread_tc(const SpreadArgs<float>& a, cudaStream_t stream);
 // Status word of the tensor-core spreading: nonzero once one of its bounded waits gave up
@@ -114,6 +117,8 @@ template <typename T>
 void launch_interp(const InterpArgs<T>& a, cudaStream_t stream);
 template <typename T>
 void launch_interp_zwin(const InterpArgs<T>& a, cudaStream_t stream);
+template <typename T>
+void launch_interp_strip(const InterpArgs<T>& a, cudaStream_t stream);
 
 // ---- z-window kernels over many transforms (zwin.cu) --------------------------------------------
 // Plane chunks of the z-window kernels: each (x, y) column is cut into `count` chunks of `len`

@@ -37,6 +37,11 @@ CoordPtrs<T> coords(int dim, const void* const* loc) {
   return c;
 }
 
+// Order of the bins of a plan's points (make_geom).
+int bin_order(int method, bool strips) {
+  return strips ? kBinsStrips : (method >= 3 ? kBinsPlaneFastest : kBinsXFastest);
+}
+
 void check_strides(int dim, const i64* modes, const i64* strides) {
   if (!strides) throw_input("null strides");
   for (int d = 0; d < dim; ++d) {
@@ -145,8 +150,13 @@ public:
       corr_[d].set_allocator(alloc_);
       upload(corr_[d], deconv_factors(kp_, nf_[d]), stream_);
     }
-    choose_tile(dim, kp_.w, sizeof(cplx_t<T>), nf_, opt.tile, method_, tile_);
-    geom_ = make_geom(dim, kp_.w, nf_, tile_, nullptr, nullptr, method_ >= 3);
+    const bool strips = use_strips(dim, kp_.w, sizeof(cplx_t<T>), nf_, opt.tile, method_);
+    if (strips) {
+      strip_tile(dim, kp_.w, sizeof(cplx_t<T>), nf_, 0, tile_);
+    } else {
+      choose_tile(dim, kp_.w, sizeof(cplx_t<T>), nf_, opt.tile, method_, tile_);
+    }
+    geom_ = make_geom(dim, kp_.w, nf_, tile_, nullptr, nullptr, bin_order(method_, strips));
     set_points(M, loc);
   }
 
@@ -502,7 +512,13 @@ public:
       quad_.z[i] = quad.z[i];
       quad_.kv[i] = quad.kv[i];
     }
-    choose_tile(dim_, kp_.w, sizeof(cplx_t<T>), nf1_, opt_.tile, method_, in_tile_);
+    in_strips_ = use_strips(dim_, kp_.w, sizeof(cplx_t<T>), nf1_, opt_.tile, method_);
+    if (in_strips_) {
+      strip_tile(dim_, kp_.w, sizeof(cplx_t<T>), nf1_, 0, in_tile_);
+    } else {
+      choose_tile(dim_, kp_.w, sizeof(cplx_t<T>), nf1_, opt_.tile, method_, in_tile_);
+    }
+    // the output points' strips depend on their number 
     choose_tile(dim_, kp_.w, sizeof(cplx_t<T>), nfft_, opt_.tile, method_, out_tile_);
     NNB_CUDA(cudaStreamSynchronize(stream_));
   }
@@ -524,7 +540,8 @@ public:
     }
     double scale[3];
     for (int d = 0; d < 3; ++d) scale[d] = d < dim_ ? 1.0 / gamma_[d] : 1.0;
-    const BinGeom g = make_geom(dim_, kp_.w, nf1_, in_tile_, C_, scale, method_ >= 3);
+    const BinGeom g = make_geom(dim_, kp_.w, nf1_, in_tile_, C_, scale,
+                                bin_order(method_, in_strips_));
     ScopedStage st(timer_, stream_, NNB_STAGE_BIN);
     in_points_.build(g, x, M, stream_);
   }
@@ -535,7 +552,10 @@ public:
     const CoordPtrs<T> s = coords<T>(dim_, pts);
     double scale[3];
     for (int d = 0; d < 3; ++d) scale[d] = d < dim_ ? gamma_[d] * h_[d] : 1.0;
-    const BinGeom g = make_geom(dim_, kp_.w, nfft_, out_tile_, D_, scale, method_ >= 3);
+    int tile[3] = {out_tile_[0], out_tile_[1], out_tile_[2]};
+    const bool strips = method_ == 1 && dim_ < 3 && !(opt_.tile[0] > 0);
+    if (strips) strip_tile(dim_, kp_.w, sizeof(cplx_t<T>), nfft_, K > 0 ? K : 1, tile);
+    const BinGeom g = make_geom(dim_, kp_.w, nfft_, tile, D_, scale, bin_order(method_, strips));
     {
       ScopedStage st(timer_, stream_, NNB_STAGE_BIN);
       out_points_.build(g, s, K, stream_);
@@ -651,6 +671,7 @@ private:
   double C_[3] = {0, 0, 0}, D_[3] = {0, 0, 0};
   double gamma_[3] = {1, 1, 1}, h_[3] = {1, 1, 1};
   int in_tile_[3] = {1, 1, 1};
+  bool in_strips_ = false;  // the input points are ordered along strips
   int out_tile_[3] = {1, 1, 1};
   int method_ = kDefaultMethod;
   i64 spread_cells_ = 0;

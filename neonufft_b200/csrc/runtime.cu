@@ -514,12 +514,34 @@ void choose_tile(int dim, int w, size_t complex_bytes, const i64* nf, const int*
   }
 }
 
+bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
+                int method) {
+  if (method != 1 || dim > 2 || (requested && requested[0] > 0)) return false;
+  // one bin per strip and row: beyond 2^26 bins (256 MB of counts) the slab tiles stay cheaper
+  if (dim == 1) return nf[0] <= (i64(1) << 26);
+  const i64 tx = strip_width(complex_bytes / 2, w);
+  return nf[1] <= 0x7fffffff && (nf[0] + tx - 1) / tx <= (i64(1) << 26) / nf[1];
+}
+
+void strip_tile(int dim, int w, size_t complex_bytes, const i64* nf, i64 interp_only_points,
+                int* tile) {
+  tile[0] = dim == 1 ? 1 : strip_width(complex_bytes / 2, w);
+  tile[1] = tile[2] = 1;
+  if (interp_only_points <= 0) return;
+  const int grow = dim - 1;  // 1D: more cells, 2D: more rows
+  i64 bins = dim == 1 ? nf[0] : (nf[0] + tile[0] - 1) / tile[0] * nf[1];
+  for (; (bins > interp_only_points / 2 && tile[grow] < 64) || bins > (i64(1) << 26); bins /= 2) {
+    tile[grow] *= 2;
+  }
+}
+
 BinGeom make_geom(int dim, int w, const i64* nf, const int* tile, const double* offset,
-                  const double* scale, int zmajor) {
+                  const double* scale, int order) {
   BinGeom g{};
   g.dim = dim;
   g.w = w;
-  g.zmajor = (dim == 3 && zmajor) ? 1 : 0;
+  g.zmajor = (dim == 3 && order == kBinsPlaneFastest) ? 1 : 0;
+  g.strip = (dim < 3 && order == kBinsStrips) ? 1 : 0;
   g.total_tiles = 1;
   for (int d = 0; d < 3; ++d) {
     if (d < dim) {

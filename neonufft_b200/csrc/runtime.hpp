@@ -192,8 +192,19 @@ int choose_method(int dim, int w, int requested, bool single);
 void choose_tile(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
                  int method, int* tile);
 
-// zmajor: order the bins plane-fastest (method 3).
+// Whether a 1D or 2D point set is ordered along strips (strip.cu): method 1 without an explicit
+// tile, where the strips' bins stay few enough to count.
+bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
+                int method);
+
+// Tile of a strip-ordered point set: bins of one row (spreading walks the points row by row), or
+// for a set of M points that is only interpolated at, enough rows for about two points per bin.
+void strip_tile(int dim, int w, size_t complex_bytes, const i64* nf, i64 interp_only_points,
+                int* tile);
+
+// order: kBinsXFastest, kBinsPlaneFastest (methods 3 to 5) or kBinsStrips.
+enum { kBinsXFastest = 0, kBinsPlaneFastest = 1, kBinsStrips = 2 };
 BinGeom make_geom(int dim, int w, const i64* nf, const int* tile, const double* offset,
-                  const double* scale, int zmajor = 0);
+                  const double* scale, int order = kBinsXFastest);
 
 }  // namespace nnb

@@ -454,6 +454,7 @@ size_t spread_smem_bytes(int dim, int w, const int* tile, size_t complex_bytes, 
 template <typename T>
 void launch_spread(const SpreadArgs<T>& a, cudaStream_t stream) {
   if (a.g.total_tiles <= 0 || a.batch <= 0) return;
+  if (a.g.strip) return launch_spread_strip<T>(a, stream);
   if (a.method == 3 || a.method == 4) return launch_spread_zwin<T>(a, stream);
   if (a.method == 5) {
     if constexpr (std::is_same<T, float>::value) return launch_spread_tc(a, stream);

@@ -1,0 +1,69 @@
+"""1D and 2D transforms on strip-sorted points (method 1 with the automatic tile, csrc/strip.cu)
+against the FP64 direct sums and the thread-per-point method, at the sizes where its runs, batches,
+strips and windows end."""
+import numpy as np
+import pytest
+
+from test_gpu_methods import direct, run_t12, width_bound
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(engine, cuda, oracle, dtype, w, type_, pts, modes, **opt):
+    rng = np.random.default_rng(w)
+    M = len(pts[0])
+    n_in = M if type_ == 1 else int(np.prod(modes))
+    inp = rng.standard_normal(n_in) + 1j * rng.standard_normal(n_in)
+    out, info = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w, **opt)
+    assert info["spread_method"] == 1
+    tpp, _ = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w, spread_method=2,
+                     **opt)
+    ref = direct(oracle, type_, 1, pts, inp, modes, dtype)
+    # the same kernel and grid: another order of the sums. Single precision: the values are sums
+    # of up to M w^d terms of relative error 6e-8 (measured 2e-7); double: 1e-16 (measured 1e-15)
+    assert oracle.rel_l2(out, tpp) < (2e-6 if dtype == "float32" else 1e-13)
+    if opt.get("upsampfac", 2.0) == 2.0:
+        assert oracle.rel_l2(out, ref) < width_bound(dtype, w)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", list(range(2, 17)))
+@pytest.mark.parametrize("type_", [1, 2])
+@pytest.mark.parametrize("modes", [[41], [20, 17]])
+def test_widths(dtype, w, type_, modes, cuda, engine, oracle):
+    """Every width; grids of a few windows (strips and rows wrap around)."""
+    rng = np.random.default_rng(w + type_)
+    pts = [rng.uniform(-4, 4, 777) for _ in modes]
+    _check(engine, cuda, oracle, dtype, w, type_, pts, modes)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 15, 16, 17, 255, 256, 257, 2049])
+@pytest.mark.parametrize("type_", [1, 2])
+@pytest.mark.parametrize("modes", [[3], [500], [2, 3], [61, 45]])
+def test_run_lengths(dtype, M, type_, modes, cuda, engine, oracle):
+    """Point counts around the batch, run and CTA sizes, on sparse and on tiny grids (narrower
+    than a strip's region)."""
+    rng = np.random.default_rng(M)
+    pts = [rng.uniform(-np.pi, np.pi, M) for _ in modes]
+    _check(engine, cuda, oracle, dtype, 6, type_, pts, modes)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("type_", [1, 2])
+def test_odd_grid(dtype, type_, cuda, engine, oracle):
+    """An odd fine grid (37 x 31): rows start 8-byte aligned only in single precision."""
+    rng = np.random.default_rng(3)
+    pts = [rng.uniform(-np.pi, np.pi, 3000) for _ in range(2)]
+    _check(engine, cuda, oracle, dtype, 7, type_, pts, [25, 21], upsampfac=1.5)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("type_", [1, 2])
+@pytest.mark.parametrize("modes", [[64], [40, 30]])
+def test_clusters(dtype, type_, modes, cuda, engine, oracle):
+    """Runs that lie in one cell, and runs that jump over rows, strips and the periodic edge."""
+    rng = np.random.default_rng(5)
+    pts = [np.concatenate([np.full(4000, 0.3), np.full(50, np.pi - 1e-4), np.full(50, -np.pi),
+                           rng.uniform(-np.pi, np.pi, 100)]) for _ in modes]
+    _check(engine, cuda, oracle, dtype, 6, type_, pts, modes)
