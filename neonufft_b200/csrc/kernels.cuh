@@ -89,6 +89,8 @@ template <typename T>
 void launch_spread(const SpreadArgs<T>& a, cudaStream_t stream);
 template <typename T>
 void launch_spread_zwin(const SpreadArgs<T>& a, cudaStream_t stream);
+template <typename T>
+void launch_spread_zwin_wide(const SpreadArgs<T>& a, cudaStream_t stream);
 // 1D and 2D spreading of strip-ordered points (strip.cu).
 template <typename T>
 void launch_spread_strip(const SpreadArgs<T>& a, cudaStream_t stream);
@@ -117,6 +119,8 @@ template <typename T>
 void launch_interp(const InterpArgs<T>& a, cudaStream_t stream);
 template <typename T>
 void launch_interp_zwin(const InterpArgs<T>& a, cudaStream_t stream);
+template <typename T>
+void launch_interp_zwin_wide(const InterpArgs<T>& a, cudaStream_t stream);
 template <typename T>
 void launch_interp_strip(const InterpArgs<T>& a, cudaStream_t stream);
 

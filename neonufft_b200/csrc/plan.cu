@@ -142,8 +142,8 @@ public:
     }
     kp_ = kernel_param(opt.tol, opt.upsampfac, is_single<T>(), opt.n_spread);
     if (kp_.w < 2 || kp_.w > 16) throw_internal("n_spread not in [2, 16]");
-    method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>());
     for (int d = 0; d < dim; ++d) nf_[d] = fine_grid_size(modes_[d], opt.upsampfac, kp_.w);
+    method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>(), opt.tile, nf_);
     fft_ = std::make_unique<FftGrid<T>>(alloc_, dim, nf_, sign_, stream_);
     fft_->enable_mode_pruning(modes_);
     for (int d = 0; d < dim; ++d) {
@@ -281,7 +281,9 @@ public:
   }
 
   bool fused_key(int* key) const override {
-    if (method_ != 3 || dim_ != 3 || points_.size() == 0 || tile_[1] != 8) return false;
+    if (method_ != 3 || dim_ != 3 || kp_.w > 8 || points_.size() == 0 || tile_[1] != 8) {
+      return false;
+    }
     *key = kp_.w | (tile_[0] << 8);
     return true;
   }
@@ -422,7 +424,7 @@ public:
     if (batch > 65535) throw_input("batch size above 65535");
     kp_ = kernel_param(opt.tol, opt.upsampfac, is_single<T>(), opt.n_spread);
     if (kp_.w < 2 || kp_.w > 16) throw_internal("n_spread not in [2, 16]");
-    method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>());
+    method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>(), opt.tile, nullptr);
     for (auto& c : corr_) c.set_allocator(alloc_);
   }
 
@@ -498,6 +500,7 @@ public:
       h_[d] = 2.0 * 3.14159265358979323846 / double(nf1_[d]);
       spread_cells *= nf1_[d];
     }
+    method_ = choose_method(dim_, kp_.w, opt_.spread_method, is_single<T>(), opt_.tile, nfft_);
     spread_cells_ = spread_cells;
     spread_grid_.reserve(size_t(spread_cells * batch_));
     NNB_CUDA(cudaMemsetAsync(spread_grid_.data(), 0,

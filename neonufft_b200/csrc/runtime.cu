@@ -401,7 +401,7 @@ template class PointSet<float>;
 template class PointSet<double>;
 
 // ---- tiles ----------------------------------------------------------------------------------------
-int choose_method(int dim, int w, int requested, bool single) {
+int choose_method(int dim, int w, int requested, bool single, const int* tile, const i64* nf) {
   if (requested == 3 && (dim != 3 || w > 8)) {
     throw_input("spread method 3 needs a 3D plan with kernel width <= 8");
   }
@@ -413,7 +413,9 @@ int choose_method(int dim, int w, int requested, bool single) {
   }
   if (requested < 0 || requested > 5) throw_input("spread method must be in [0, 5]");
   if (requested > 0) return requested;
-  return (dim == 3 && w <= 8) ? 3 : 1;
+  if (dim < 3) return 1;
+  if (w <= 8) return 3;
+  return (tile && tile[0] > 0) || (nf && nf[2] >= (i64(1) << 24)) ? 1 : 3;
 }
 
 void choose_tile(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,

@@ -183,9 +183,11 @@ private:
 };
 
 // Spreading / interpolation method for a plan: the requested one (validated), or the default:
-// 3 (z-window, zwin.cu) for 3D plans with n_spread <= 8, else 1 (shared-memory slabs). Method 4
-// is the z-window with tensor-core spreading (single precision, 5 <= n_spread <= 8).
-int choose_method(int dim, int w, int requested, bool single);
+// 3 (z-window, zwin.cu) for 3D plans, else 1 (strips, or shared-memory slabs). A 3D plan with
+// n_spread > 8 keeps the slabs when it names a tile or has 2^24 planes or more (nf, which may be
+// null as long as it is not known). Method 4 is the z-window with tensor-core spreading (single
+// precision, 5 <= n_spread <= 8).
+int choose_method(int dim, int w, int requested, bool single, const int* tile, const i64* nf);
 
 // Tile shape for a grid and method: explicit request (validated) or the automatic choice.
 // Method 3 uses (tx, 8, 1) tiles, tx in {4, 8}.
