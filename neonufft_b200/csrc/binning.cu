@@ -296,6 +296,35 @@ __global__ void __launch_bounds__(kScanThreads)
   if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = block_offsets[nb];
 }
 
+// The whole scan in one CTA, for counts too few to be worth three launches (one pass of the CTA:
+// 2000 counts 3.2 us against 7.9; four passes, 32768 counts, took 25 us).
+constexpr int kScanSmallThreads = 1024;
+constexpr i64 kScanSmall = kScanSmallThreads * kScanItems;
+__global__ void __launch_bounds__(kScanSmallThreads)
+    scan_small_kernel(const u32* in, i64 n, u32* out) {
+  __shared__ u64 total;
+  u64 carry = 0;
+  for (i64 off = 0; off < n; off += kScanSmallThreads * kScanItems) {
+    const i64 base = off + threadIdx.x * kScanItems;
+    u32 v[kScanItems];
+    u64 s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = (base + k < n) ? in[base + k] : 0u;
+      s += v[k];
+    }
+    u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total) + carry;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (base + k < n) out[base + k] = u32(run);
+      run += v[k];
+    }
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[n] = u32(carry);
+}
+
 // Whether a record array starts on a 32-byte boundary (a user allocator may return less), so
 // that its records take single 256-bit stores.
 bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
@@ -328,6 +357,11 @@ i64 scan_tmp_words(i64 n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream) {
   const i64 nb = (n + kScanChunk - 1) / kScanChunk;
   if (nb <= 0) return;
+  if (n <= kScanSmall) {
+    scan_small_kernel<<<1, kScanSmallThreads, 0, stream>>>(counts, n, out);
+    NNB_LAUNCH_CHECK();
+    return;
+  }
   scan_block_sums_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, tmp);
   NNB_LAUNCH_CHECK();
   scan_top_kernel<<<1, kScanThreads, 0, stream>>>(tmp, nb);

@@ -133,11 +133,11 @@ struct ZChunks {
 };
 // Chunks of `len` planes for ncols columns of nz planes (at least 4 w planes each), and the work
 // list of a plane-major point set's (column, chunk) units (zwin.cu; also used by the
-// tensor-core spreading, spread_tc.cu).
+// tensor-core spreading, spread_tc.cu). The list is built once per point set
+// (zwin_build_work_list, called when the points are binned) and read by every transform.
 ZChunks make_chunks(i64 ncols, int nz, int w);
 template <typename T>
-WorkList zwin_work_list(const BinGeom& g, const SortedPoints<T>& pts, ZChunks ch,
-                        cudaStream_t stream);
+WorkList zwin_work_list(const BinGeom& g, const SortedPoints<T>& pts, ZChunks ch);
 // One transform's share of a persistent launch: its arguments, chunks and work list.
 template <typename T>
 struct ZSpreadJob {
@@ -151,8 +151,7 @@ struct ZInterpJob {
   ZChunks ch;
   WorkList wl;
 };
-// Host-side descriptions (nothing is launched); the work lists they name are built on the
-// device by zwin_build_work_list, which must run before the persistent launch.
+// Host-side descriptions (nothing is launched).
 template <typename T>
 ZSpreadJob<T> zwin_spread_job(const SpreadArgs<T>& a);
 template <typename T>

@@ -307,7 +307,6 @@ public:
                          stream_);
       fft_->exec_from_modes(fft_->data(), stream_);
     }
-    zwin_build_work_list<T>(geom_, points_.view(), stream_);
   }
 
   void fused_post(int type, void* out, const i64* strides) override {

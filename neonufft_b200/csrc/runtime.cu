@@ -329,7 +329,7 @@ template class FftGrid<double>;
 template <typename T>
 PointSet<T>::PointSet(std::shared_ptr<DeviceAllocator> alloc)
     : rec_(alloc), counts_(alloc), bin_start_(alloc), ranks_(alloc), scan_tmp_(alloc),
-      work_start_(alloc), work_owner_(alloc), err_(alloc), checksum_(alloc) {}
+      work_start_(alloc), work_owner_(alloc), checksum_(alloc) {}
 
 template <typename T>
 void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream) {
@@ -341,22 +341,26 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   g_ = g;
   M_ = M;
   const i64 nt = g.total_tiles;
-  counts_.reserve(size_t(nt));
+  counts_.reserve(size_t(nt + 1));  // the error flag behind the counts: one memset for both
   bin_start_.reserve(size_t(nt + 1));
   scan_tmp_.reserve(size_t(scan_tmp_words(nt)));
   rec_.reserve(size_t(M));
   ranks_.reserve(size_t(M));
-  // work lists reuse counts_ and scan_tmp_ after binning (launch units never exceed the tiles)
-  work_start_.reserve(size_t(nt + 1));
-  work_owner_.reserve(size_t(nt + M / kWorkItemPoints + 2));
-  err_.reserve(1);
-  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * nt, stream));
-  NNB_CUDA(cudaMemsetAsync(err_.data(), 0, sizeof(int), stream));
-  launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err_.data(), stream);
+  // work lists reuse counts_ and scan_tmp_ after binning (launch units never exceed the tiles);
+  // strip-ordered points need none
+  if (!g.strip) {
+    work_start_.reserve(size_t(nt + 1));
+    work_owner_.reserve(size_t(nt + M / kWorkItemPoints + 2));
+  }
+  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nt + 1), stream));
+  int* err = reinterpret_cast<int*>(counts_.data() + nt);
+  launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err, stream);
   launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream);
   launch_bin_scatter<T>(g, x, M, ranks_.data(), bin_start_.data(), rec_.data(), stream);
+  // every z-window transform of these points walks the same list of work items
+  if (g.zmajor && M > 0) zwin_build_work_list<T>(g, view(), stream);
   int host_err = 0;
-  NNB_CUDA(cudaMemcpyAsync(&host_err, err_.data(), sizeof(int), cudaMemcpyDeviceToHost, stream));
+  NNB_CUDA(cudaMemcpyAsync(&host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));
 #ifdef NNB_CHECKED
   // The records' permutation must be 0 .. M - 1, each once: compare its sum and sum of squares
   // (wrapping 64-bit, as the device adds them) with the closed forms.

@@ -178,7 +178,6 @@ private:
   i64 M_ = 0;
   DevArray<PointRec<T>> rec_;
   DevArray<u32> counts_, bin_start_, ranks_, scan_tmp_, work_start_, work_owner_;
-  DevArray<int> err_;
   DevArray<unsigned long long> checksum_;  // checked build: permutation checksum of the records
 };
 

@@ -580,7 +580,7 @@ template <int W>
 void launch_spread_tc_w(const SpreadArgs<float>& a, cudaStream_t stream) {
   const i64 ncols = i64(a.g.ntiles[0]) * a.g.ntiles[1];
   const ZChunks ch = make_chunks(ncols, a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   const size_t smem = sizeof(TcShared<W>);
   // the dynamic shared-memory limit is an attribute of the function on the current device; a
   // host-side call per launch, so any device the caller switches to is covered

@@ -43,11 +43,13 @@ __global__ void __launch_bounds__(kWlThreads)
   cnt[u] = (n + cap - 1) / cap;
 }
 
+// One warp per unit: a unit that holds most of the points has many items.
 __global__ void __launch_bounds__(kWlThreads)
     owner_kernel(i64 units, const u32* start, u32* owner) {
-  const i64 u = blockIdx.x * i64(kWlThreads) + threadIdx.x;
+  const i64 u = blockIdx.x * i64(kWlThreads / 32) + (threadIdx.x >> 5);
   if (u >= units) return;
-  for (u32 i = start[u]; i < start[u + 1]; ++i) owner[i] = u32(u);
+  const u32 end = start[u + 1];
+  for (u32 i = start[u] + (threadIdx.x & 31); i < end; i += 32) owner[i] = u32(u);
 }
 
 }  // namespace
@@ -71,7 +73,9 @@ WorkList build_work_list(const UnitMap& m, const BinGeom& g, const u32* bin_star
   unit_items_kernel<<<blocks, kWlThreads, 0, stream>>>(m, g, bin_start, wl.cap, s.cnt);
   NNB_LAUNCH_CHECK();
   launch_exclusive_scan(s.cnt, s.start, m.units, s.tmp, stream);
-  owner_kernel<<<blocks, kWlThreads, 0, stream>>>(m.units, s.start, s.owner);
+  const i64 warps_per_cta = kWlThreads / 32;
+  owner_kernel<<<unsigned((m.units + warps_per_cta - 1) / warps_per_cta), kWlThreads, 0,
+                 stream>>>(m.units, s.start, s.owner);
   NNB_LAUNCH_CHECK();
   return wl;
 }

@@ -285,17 +285,13 @@ ZChunks zwin_chunks(const BinGeom& g) {
 
 // Work list of (column, chunk) units split into items of at most kWorkItemPoints points.
 template <typename T>
-WorkList zwin_work_list(const BinGeom& g, const SortedPoints<T>& pts, ZChunks ch,
-                        cudaStream_t stream) {
-  const WorkList wl = build_work_list(zwin_unit_map(g, ch), g, pts.bin_start, pts.M, pts.work,
-                                      stream);
+WorkList zwin_work_list(const BinGeom& g, const SortedPoints<T>& pts, ZChunks ch) {
+  const WorkList wl = describe_work_list(zwin_unit_map(g, ch), pts.M, pts.work);
   if (wl.grid > 0x7fffffffll) throw_input("grid too large");
   return wl;
 }
-template WorkList zwin_work_list<float>(const BinGeom&, const SortedPoints<float>&, ZChunks,
-                                         cudaStream_t);
-template WorkList zwin_work_list<double>(const BinGeom&, const SortedPoints<double>&, ZChunks,
-                                          cudaStream_t);
+template WorkList zwin_work_list<float>(const BinGeom&, const SortedPoints<float>&, ZChunks);
+template WorkList zwin_work_list<double>(const BinGeom&, const SortedPoints<double>&, ZChunks);
 
 namespace {
 
@@ -304,7 +300,7 @@ void launch_spread_zwin_tw(const SpreadArgs<T>& a, cudaStream_t stream) {
   using S = ZShape<T, W, TX, TY>;
   const i64 ncols = i64(a.g.ntiles[0]) * a.g.ntiles[1];
   const ZChunks ch = make_chunks(ncols, a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   // Single precision with the default or 4-row tiles spreads two strength vectors per pass
   // when there are several (the second vector costs its FMAs only).
   constexpr bool kPairs = std::is_same<T, float>::value && TX == 4 && (TY == 8 || TY == 4);
@@ -326,7 +322,7 @@ void launch_interp_zwin_tw(const InterpArgs<T>& a, cudaStream_t stream) {
   using S = ZShape<T, W, TX, TY>;
   const i64 ncols = i64(a.g.ntiles[0]) * a.g.ntiles[1];
   const ZChunks ch = make_chunks(ncols, a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   interp_zwin_kernel<T, W, TX, TY><<<unsigned(wl.grid), S::NT, 0, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
 }
@@ -429,7 +425,7 @@ template <int W>
 void launch_spread_zmma_w(const SpreadArgs<float>& a, cudaStream_t stream) {
   const i64 ncols = i64(a.g.ntiles[0]) * a.g.ntiles[1];
   const ZChunks ch = make_chunks(ncols, a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   dim3 grid{unsigned(wl.grid), unsigned(a.batch), 1u};
   spread_zmma_kernel<W><<<grid, 128, 0, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
@@ -521,8 +517,9 @@ ZInterpJob<T> zwin_interp_job(const InterpArgs<T>& a) {
 
 template <typename T>
 void zwin_build_work_list(const BinGeom& g, const SortedPoints<T>& pts, cudaStream_t stream) {
-  check_zwin_geom(g);
-  (void)zwin_work_list(g, pts, zwin_chunks(g), stream);
+  if (g.dim != 3 || !g.zmajor) throw_internal("z-window work lists need plane-major points");
+  (void)build_work_list(zwin_unit_map(g, zwin_chunks(g)), g, pts.bin_start, pts.M, pts.work,
+                        stream);
 }
 
 template <typename T>

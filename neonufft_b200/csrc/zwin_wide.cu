@@ -20,7 +20,7 @@ template <typename T, int W>
 void spread_wide_w(const SpreadArgs<T>& a, cudaStream_t stream) {
   using S = ZShape<T, W, kWideTx, kWideTy>;
   const ZChunks ch = make_chunks(i64(a.g.ntiles[0]) * a.g.ntiles[1], a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   dim3 grid{unsigned(wl.grid), unsigned(a.batch), 1u};
   spread_zwin_kernel<T, W, kWideTx, kWideTy><<<grid, S::NT, 0, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
@@ -34,7 +34,7 @@ void interp_wide_w(const InterpArgs<T>& a, cudaStream_t stream) {
   // Per device and cheap; set on every launch so that multi-device processes stay correct.
   NNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const ZChunks ch = make_chunks(i64(a.g.ntiles[0]) * a.g.ntiles[1], a.g.ntiles[2], W);
-  const WorkList wl = zwin_work_list(a.g, a.pts, ch, stream);
+  const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   kern<<<unsigned(wl.grid), S::NT, smem, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
 }
