@@ -83,6 +83,7 @@ struct SpreadArgs {
   int batch;
   T beta;
   T c;
+  EsPoly<T> es;
   int method;  // 1: warp-private slabs, 2: thread per point, 3: z-window, 4: z-window on tensor cores (zwin.cu)
 };
 template <typename T>
@@ -113,6 +114,7 @@ struct InterpArgs {
   cplx_t<T>* out;              // original point order
   T beta;
   T c;
+  EsPoly<T> es;
   int method;  // 1: warp per point, 2: thread per point, 3: z-window (zwin.cu)
 };
 template <typename T>

@@ -175,6 +175,57 @@ double es_kernel(const KernelParam& kp, double x) {
   return std::exp(kp.beta * (std::sqrt(arg) - 1.0));
 }
 
+template <typename T>
+EsPoly<T> es_poly(const KernelParam& kp) {
+  constexpr int NE = EsPoly<T>::NE, NO = EsPoly<T>::NO, n = NE + NO;
+  const long double pi = 3.141592653589793238462643383279502884L;
+  EsPoly<T> p{};
+  auto phi = [&](long double x) {
+    const long double arg = 1.0L - static_cast<long double>(kp.c) * x * x;
+    return arg > 0.0L ? std::exp(static_cast<long double>(kp.beta) * (std::sqrt(arg) - 1.0L))
+                      : 0.0L;
+  };
+  long double edge = 0.0L, inner = 0.0L;  // largest errors of the fits
+  for (int k = 0; k < (kp.w + 1) / 2; ++k) {
+    const long double centre = k - kp.w / 2.0L + 0.5L;
+    // Chebyshev coefficients from the n zeros of T_n, then monomials
+    long double f[n], a[n];
+    for (int j = 0; j < n; ++j) f[j] = phi(centre + 0.5L * std::cos(pi * (j + 0.5L) / n));
+    for (int m = 0; m < n; ++m) {
+      a[m] = 0.0L;
+      for (int j = 0; j < n; ++j) a[m] += f[j] * std::cos(pi * m * (j + 0.5L) / n);
+      a[m] *= (m ? 2.0L : 1.0L) / n;
+    }
+    long double mono[n] = {}, t0[n] = {}, t1[n] = {};  // sum, T_{m-1}, T_m
+    t0[0] = 1.0L;
+    t1[1] = 1.0L;
+    for (int i = 0; i < n; ++i) mono[i] = a[0] * t0[i] + a[1] * t1[i];
+    for (int m = 2; m < n; ++m) {
+      long double t2[n];
+      for (int i = 0; i < n; ++i) t2[i] = (i ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+      for (int i = 0; i < n; ++i) {
+        mono[i] += a[m] * t2[i];
+        t0[i] = t1[i];
+        t1[i] = t2[i];
+      }
+    }
+    for (int i = 0; i < n; ++i) (i % 2 ? p.o[k][i / 2] : p.e[k][i / 2]) = T(mono[i]);
+    for (int j = 0; j <= 100; ++j) {
+      const long double t = -1.0L + 0.02L * j;
+      long double v = 0.0L;
+      for (int i = n - 1; i >= 0; --i) v = v * t + mono[i];
+      long double& worst = k == 0 ? edge : inner;
+      worst = std::max(worst, std::abs(v - phi(centre + 0.5L * t)));
+    }
+  }
+  const long double limit = sizeof(T) == 4 ? 3e-8L : 2e-16L;
+  p.mode = inner > (sizeof(T) == 4 ? limit : 1e-15L) ? kEsAllExact
+                                                     : (edge > limit ? kEsExactEdges : kEsAllPoly);
+  return p;
+}
+template EsPoly<float> es_poly<float>(const KernelParam&);
+template EsPoly<double> es_poly<double>(const KernelParam&);
+
 PhiHatQuad phi_hat_quadrature(const KernelParam& kp) {
   // The kernel is even, so only the q nodes on (0, 1] of a 2q-node rule are used:
   // integral_{-w/2}^{w/2} phi(z) cos(xi z) dz = w * sum_q W_q phi(z_q w/2) cos(xi z_q w/2).

@@ -13,6 +13,8 @@
 #include <cstdint>
 #include <vector>
 
+#include "es_poly.hpp"
+
 namespace nnb {
 
 struct KernelParam {
@@ -62,6 +64,11 @@ PhiHatQuad phi_hat_quadrature(const KernelParam& kp);
 
 // ES kernel value in double precision (with the plan's rounded beta and c).
 double es_kernel(const KernelParam& kp, double x);
+
+// Polynomials of the kernel's pieces, and which of them are accurate enough to be used: within
+// 3e-8 (T = float) or 2e-16 (double) of the kernel's peak, else that piece stays with the formula.
+template <typename T>
+EsPoly<T> es_poly(const KernelParam& kp);
 
 // corr[k] = (-1)^k / phi_hat(2 pi k / nf), k = 0 .. nf/2 (nf/2 + 1 values).
 std::vector<double> deconv_factors(const KernelParam& kp, std::int64_t nf);

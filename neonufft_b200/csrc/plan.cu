@@ -142,6 +142,7 @@ public:
     }
     kp_ = kernel_param(opt.tol, opt.upsampfac, is_single<T>(), opt.n_spread);
     if (kp_.w < 2 || kp_.w > 16) throw_internal("n_spread not in [2, 16]");
+    es_ = es_poly<T>(kp_);
     for (int d = 0; d < dim; ++d) nf_[d] = fine_grid_size(modes_[d], opt.upsampfac, kp_.w);
     method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>(), opt.tile, nf_);
     fft_ = std::make_unique<FftGrid<T>>(alloc_, dim, nf_, sign_, stream_);
@@ -351,6 +352,7 @@ private:
     a.batch = 1;
     a.beta = T(kp_.beta);
     a.c = T(kp_.c);
+    a.es = es_;
     a.method = method_;
     return a;
   }
@@ -364,6 +366,7 @@ private:
     a.out = static_cast<cplx_t<T>*>(out);
     a.beta = T(kp_.beta);
     a.c = T(kp_.c);
+    a.es = es_;
     a.method = method_;
     return a;
   }
@@ -387,6 +390,7 @@ private:
   int sign_;
   cudaStream_t stream_;
   KernelParam kp_;
+  EsPoly<T> es_{};
   i64 modes_[3];
   i64 nf_[3];
   int tile_[3] = {1, 1, 1};
@@ -423,6 +427,7 @@ public:
     if (batch > 65535) throw_input("batch size above 65535");
     kp_ = kernel_param(opt.tol, opt.upsampfac, is_single<T>(), opt.n_spread);
     if (kp_.w < 2 || kp_.w > 16) throw_internal("n_spread not in [2, 16]");
+    es_ = es_poly<T>(kp_);
     method_ = choose_method(dim, kp_.w, opt.spread_method, is_single<T>(), opt.tile, nullptr);
     for (auto& c : corr_) c.set_allocator(alloc_);
   }
@@ -587,6 +592,7 @@ public:
     a.batch = int(batch_);
     a.beta = T(kp_.beta);
     a.c = T(kp_.c);
+    a.es = es_;
     a.method = method_;
     launch_spread<T>(a, stream_);
   }
@@ -625,6 +631,7 @@ public:
       a.out = static_cast<cplx_t<T>*>(out) + b * bdist;
       a.beta = T(kp_.beta);
       a.c = T(kp_.c);
+      a.es = es_;
       a.method = method_;
       launch_interp<T>(a, stream_);
     }
@@ -668,6 +675,7 @@ private:
   i64 batch_;
   cudaStream_t stream_;
   KernelParam kp_;
+  EsPoly<T> es_{};
   i64 nf1_[3] = {1, 1, 1};
   i64 nfft_[3] = {1, 1, 1};
   double C_[3] = {0, 0, 0}, D_[3] = {0, 0, 0};

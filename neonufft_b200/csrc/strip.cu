@@ -191,14 +191,15 @@ __global__ void __launch_bounds__(32 * kStripWarps)
 #pragma unroll
         for (int i = 0; i < int(S::KXN * sizeof(T) / 16); ++i) z[i] = make_float4(0, 0, 0, 0);
         T* dst = sl.kx + unsigned(x0) % unsigned(S::TX);
+        T wt[W];
+        es_weights<W>(rec.frac[0], a.es, a.beta, a.c, wt);
 #pragma unroll
-        for (int i = 0; i < W; ++i) dst[i] = es_eval_fast<T>(rec.frac[0] + T(i), a.beta, a.c);
+        for (int i = 0; i < W; ++i) dst[i] = wt[i];
       }
-      const T fw = rec.frac[DIM - 1];
+      T wt[W];
+      es_weights<W>(rec.frac[DIM - 1], a.es, a.beta, a.c, wt);
 #pragma unroll
-      for (int i = 0; i < RY; ++i) {
-        sl.ky[i] = i < W ? es_eval_fast<T>(fw + T(i), a.beta, a.c) : T(0);
-      }
+      for (int i = 0; i < RY; ++i) sl.ky[i] = i < W ? wt[i < W ? i : 0] : T(0);
       sl.v = val;
       sl.row = DIM == 2 ? y0 : x0;
       sl.strip = DIM == 2 ? int(unsigned(x0) / unsigned(S::TX)) : 0;
@@ -259,14 +260,14 @@ __global__ void __launch_bounds__(kStripInterpThreads)
   const i64 nfx = a.g.nf[0];
   [[maybe_unused]] const i64 cells = a.g.nf[0] * a.g.nf[1];
   const C* __restrict__ grid = a.grid;
-  T kx[W];
-#pragma unroll
-  for (int k = 0; k < W; ++k) kx[k] = es_eval_fast<T>(rec.frac[0] + T(k), a.beta, a.c);
-  T sx = 0, sy = 0;
   constexpr int NR = DIM == 1 ? 1 : W;
+  T kx[W], ky[NR];
+  es_weights<W>(rec.frac[0], a.es, a.beta, a.c, kx);
+  if constexpr (DIM == 2) es_weights<W>(rec.frac[1], a.es, a.beta, a.c, ky);
+  T sx = 0, sy = 0;
   const int ny = int(a.g.nf[1]);
   const bool inside = i64(x0) + W <= nfx;  // the cells of a row are consecutive
-#pragma unroll 2
+#pragma unroll
   for (int dy = 0; dy < NR; ++dy) {
     int y = y0 + dy;
     if (DIM == 2 && y >= ny) y -= ny;
@@ -296,9 +297,8 @@ __global__ void __launch_bounds__(kStripInterpThreads)
       }
     }
     if constexpr (DIM == 2) {
-      const T ky = es_eval_fast<T>(rec.frac[1] + T(dy), a.beta, a.c);
-      sx += ky * rx;
-      sy += ky * ry;
+      sx += ky[dy] * rx;
+      sy += ky[dy] * ry;
     } else {
       sx = rx;
       sy = ry;

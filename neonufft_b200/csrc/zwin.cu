@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(128) spread_zmma_kernel(SpreadArgs<float> a, Z
       }
       stage_warp<float, W, TX, true>(slots[k & 1] + th.warp * PW + c0,
                                      a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
-                                     min(count - c0, 16), in, a.prephase, a.beta, a.c, th.lane,
+                                     min(count - c0, 16), in, a.prephase, a.es, a.beta, a.c, th.lane,
                                      a.pts.M);
     }
   };

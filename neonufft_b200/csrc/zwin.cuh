@@ -119,11 +119,15 @@ struct alignas(16) ZSlot
 // (2p, 2p + 1) fills point p's slot with the same instruction stream: the even lane kx and the
 // first half of kz, the odd lane ky and the second half, each zeroing half of the contiguous
 // kx / ky arrays first, so all 32 lanes evaluate kernel values.
-template <typename T, int W, int TX, bool SPREAD, int TY = 8>
+//
+// POLY: kernel values by the polynomials of the pieces; double precision gives each lane of the
+// pair its half of kz (single precision measured slower that way: 1.98 against 1.86 ms per 1e7
+// points) while both evaluate all of kz in single.
+template <typename T, int W, int TX, bool SPREAD, int TY = 8, bool POLY = true>
 __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const PointRec<T>* recs,
                                            int count, const cplx_t<T>* in,
-                                           const cplx_t<T>* prephase, T beta, T c, int lane,
-                                           i64 num, const cplx_t<T>* in2 = nullptr,
+                                           const cplx_t<T>* prephase,
+                                           const EsPoly<T>& es, T beta, T c, int lane, i64 num, const cplx_t<T>* in2 = nullptr,
                                            cplx_t<T>* v2_out = nullptr) {
   using S = ZShape<T, W, TX, TY>;
   using C = cplx_t<T>;
@@ -173,13 +177,36 @@ __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const Poi
     const int lx = int(loc & 0xFu);
     const int ly = int((loc >> 4) & 0xFu);
     T* dst = h ? sl.ky + ly : sl.kx + lx;
-    const T f = h ? fy : fx;
+    if constexpr (!POLY) {
+      const T f = h ? fy : fx;
 #pragma unroll
-    for (int k = 0; k < W; ++k) dst[k] = es_eval_fast<T>(f + T(k), beta, c);
+      for (int k = 0; k < W; ++k) dst[k] = es_eval_fast<T>(f + T(k), beta, c);
 #pragma unroll
-    for (int i = 0; i < S::RZS / 2; ++i) {
-      const int k = h * (S::RZS / 2) + i;
-      sl.kz[k] = k < W ? es_eval_fast<T>(fz + T(k), beta, c) : T(0);
+      for (int i = 0; i < S::RZS / 2; ++i) {
+        const int k = h * (S::RZS / 2) + i;
+        sl.kz[k] = k < W ? es_eval_fast<T>(fz + T(k), beta, c) : T(0);
+      }
+    } else {
+      T wt[W];
+      es_weights<W>(h ? fy : fx, es, beta, c, wt);
+#pragma unroll
+      for (int k = 0; k < W; ++k) dst[k] = wt[k];
+      if constexpr (sizeof(T) == 8) {
+        es_half<W>(fz, h, es, beta, c, [&](int k, T v) { sl.kz[k] = v; });
+        if (h) {
+#pragma unroll
+          for (int k = W; k < S::RZS; ++k) sl.kz[k] = T(0);
+        }
+      } else {
+        es_weights<W>(fz, es, beta, c, wt);
+#pragma unroll
+        for (int i = 0; i < S::RZS / 2; ++i) {
+          constexpr int H = S::RZS / 2;
+          const T lo = i < W ? wt[i < W ? i : 0] : T(0);
+          const T hi = H + i < W ? wt[H + i < W ? H + i : 0] : T(0);
+          sl.kz[h * H + i] = h ? hi : lo;
+        }
+      }
     }
     if (h == 0) {
       sl.v = C{vx, vy};
@@ -356,6 +383,9 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
     dirty = false;
   };
 
+  // One vector in single precision keeps the formula: with the polynomials ptxas takes 96 instead
+  // of 55 registers and 1e8 points on 480^3 cells 23.5 instead of 16.5 ms (20.2 capped at 64).
+  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || NV > 1;
   const u32 npts = cta.pend - cta.pbeg;
   const int nbatch = int((npts + S::BATCH - 1) / S::BATCH);
   auto stage = [&](int k) {
@@ -369,9 +399,9 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
         break;
       }
       // NV = 2: the second vector's strengths at the same points (zeros when it is missing)
-      stage_warp<T, W, TX, true, TY>(slots[k & 1] + th.warp * PW + c0,
+      stage_warp<T, W, TX, true, TY, kPoly>(slots[k & 1] + th.warp * PW + c0,
                                  a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
-                                 min(count - c0, 16), in, a.prephase, a.beta, a.c, th.lane,
+                                 min(count - c0, 16), in, a.prephase, a.es, a.beta, a.c, th.lane,
                                  a.pts.M, NV > 1 && has2 ? in + a.in_bdist : nullptr,
                                  NV > 1 ? sh.v2[k & 1] + th.warp * PW + c0 : nullptr);
     }
@@ -506,8 +536,11 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
   flush(cur + dz);  // the rest of the window
 }
 
+// Double precision is held to 100 registers (5 CTAs of 128 threads): uncapped, ptxas takes 106
+// and 3e6 clustered points spread in 1.59 instead of 1.19 ms.
 template <typename T, int W, int TX, int TY>
-__global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT)
+__global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT,
+                                  sizeof(T) == 8 && TX == 4 ? 65536 / (ZShape<T, W, TX, TY>::NT * 100) : 0)
     spread_zwin_kernel(const __grid_constant__ SpreadArgs<T> a, ZChunks ch,
                        const __grid_constant__ WorkList wl) {
   __shared__ ZSpreadShared<T, W, TX, TY> sh;
@@ -620,7 +653,7 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
       }
       stage_warp<T, W, TX, false, TY>(slots[k & 1] + th.warp * PW + c0,
                                   a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
-                                  min(count - c0, 16), nullptr, nullptr, a.beta, a.c, th.lane,
+                                  min(count - c0, 16), nullptr, nullptr, a.es, a.beta, a.c, th.lane,
                                   a.pts.M);
     }
   };

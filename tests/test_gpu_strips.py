@@ -29,11 +29,12 @@ def _check(engine, cuda, oracle, dtype, w, type_, pts, modes, **opt):
 @pytest.mark.parametrize("dtype", ["float32", "float64"])
 @pytest.mark.parametrize("w", list(range(2, 17)))
 @pytest.mark.parametrize("type_", [1, 2])
-@pytest.mark.parametrize("modes", [[41], [20, 17]])
-def test_widths(dtype, w, type_, modes, cuda, engine, oracle):
-    """Every width; grids of a few windows (strips and rows wrap around)."""
+@pytest.mark.parametrize("modes,M", [([41], 777), ([20, 17], 777), ([20, 17], 80)])
+def test_widths(dtype, w, type_, modes, M, cuda, engine, oracle):
+    """Every width; grids of a few windows (strips and rows wrap around); 80 points on 40 x 34
+    cells are spread one by one, 777 through windows."""
     rng = np.random.default_rng(w + type_)
-    pts = [rng.uniform(-4, 4, 777) for _ in modes]
+    pts = [rng.uniform(-4, 4, M) for _ in modes]
     _check(engine, cuda, oracle, dtype, w, type_, pts, modes)
 
 
@@ -51,10 +52,11 @@ def test_run_lengths(dtype, M, type_, modes, cuda, engine, oracle):
 
 @pytest.mark.parametrize("dtype", ["float32", "float64"])
 @pytest.mark.parametrize("type_", [1, 2])
-def test_odd_grid(dtype, type_, cuda, engine, oracle):
+@pytest.mark.parametrize("M", [60, 3000])
+def test_odd_grid(dtype, type_, M, cuda, engine, oracle):
     """An odd fine grid (37 x 31): rows start 8-byte aligned only in single precision."""
     rng = np.random.default_rng(3)
-    pts = [rng.uniform(-np.pi, np.pi, 3000) for _ in range(2)]
+    pts = [rng.uniform(-np.pi, np.pi, M) for _ in range(2)]
     _check(engine, cuda, oracle, dtype, 7, type_, pts, [25, 21], upsampfac=1.5)
 
 
@@ -67,3 +69,33 @@ def test_clusters(dtype, type_, modes, cuda, engine, oracle):
     pts = [np.concatenate([np.full(4000, 0.3), np.full(50, np.pi - 1e-4), np.full(50, -np.pi),
                            rng.uniform(-np.pi, np.pi, 100)]) for _ in modes]
     _check(engine, cuda, oracle, dtype, 6, type_, pts, modes)
+
+
+def spectrum_ratio(beta, w, upsampfac):
+    x = np.linspace(-w / 2, w / 2, 20001)
+    phi = np.exp(beta * (np.sqrt(np.maximum(0, 1 - 4 * x * x / w ** 2)) - 1))
+    return phi.sum() / (phi * np.cos(np.pi / upsampfac * x)).sum()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", [2, 3, 7, 8, 11])
+@pytest.mark.parametrize("upsampfac", [1.25, 2.0, 8.0])
+@pytest.mark.parametrize("type_", [1, 2])
+@pytest.mark.parametrize("modes", [[41], [12, 10, 9]])
+def test_kernel_polynomials(dtype, w, upsampfac, type_, modes, cuda, engine, oracle):
+    """Kernel values by polynomials (the default kernels) against the formula (method 2), over the
+    shapes of the kernel: the smallest upsampling leaves the largest edge value, the largest the
+    steepest pieces (w = 3 then stays with the formula in single precision)."""
+    rng = np.random.default_rng(w)
+    pts = [rng.uniform(-np.pi, np.pi, 500) for _ in modes]
+    n_in = 500 if type_ == 1 else int(np.prod(modes))
+    inp = rng.standard_normal(n_in) + 1j * rng.standard_normal(n_in)
+    a, _ = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w, upsampfac=upsampfac)
+    b, info = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w,
+                      upsampfac=upsampfac, spread_method=2)
+    assert info["spread_method"] == 2
+    # Single precision: a weight is off by up to 3e-7 of its value (the formula's square root is
+    # rounded before it is multiplied by beta), and the deconvolution scales the outermost modes up
+    # by phi_hat(0) / phi_hat(pi / upsampfac), 153 at w = 11 and upsampling 1.25. Double: 1e-15.
+    up = spectrum_ratio(info["es_beta"], w, upsampfac)
+    assert oracle.rel_l2(a, b) < (3e-7 * max(10, up) if dtype == "float32" else 1e-15 * max(100, up))
