@@ -28,6 +28,7 @@
 // grid, w = 6, single: spreading 579 -> 187 us, interpolation 901 -> 69 us; 5e6 points on 4e5
 // cells in 1D, w = 10, double: 888 -> 302 us and 1476 -> 152 us. Both are now bound by
 // instruction issue, half of it the kernel values.
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -247,6 +248,113 @@ __global__ void __launch_bounds__(32 * kStripWarps)
   flush(i64(cur) + dz);
 }
 
+// 2D spreading of points so sparse that a window's rows would be flushed after a point or two: the
+// warp's lanes add a point's footprint to the grid directly, neighbouring lanes neighbouring
+// cells, so that one atomic instruction covers whole sectors of several rows. An element is an
+// aligned pair of cells (16 bytes) in single precision, a real or imaginary part in double (there
+// are no vector atomics for doubles).
+template <typename T, int W>
+struct SparseShape {
+  static constexpr bool SINGLE = sizeof(T) == 4;
+  static constexpr int PER_ROW = SINGLE ? W / 2 + 1 : 2 * W;  // elements per footprint row
+  static constexpr int ELEMS = W * PER_ROW;
+  static constexpr int KXN = SINGLE ? 2 * PER_ROW : W;        // staged kx values
+};
+template <typename T, int W>
+struct SparseSlot {
+  T kx[SparseShape<T, W>::KXN];  // single: from the aligned pair that holds the first cell
+  T ky[W];
+  cplx_t<T> v;
+  int x0, y0;
+};
+
+template <typename T, int W>
+__global__ void __launch_bounds__(32 * kStripWarps)
+    spread_sparse_kernel(const __grid_constant__ SpreadArgs<T> a, bool aligned) {
+  using S = SparseShape<T, W>;
+  using C = cplx_t<T>;
+  __shared__ SparseSlot<T, W> slots[kStripWarps][32];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const i64 M = a.pts.M;
+  const i64 first = (i64(blockIdx.x) * kStripWarps + warp) * 32;
+  if (first >= M) return;
+  const int count = int(min(i64(32), M - first));
+  const C* __restrict__ in = a.in + i64(blockIdx.y) * a.in_bdist;
+  C* grid = a.grid + i64(blockIdx.y) * a.grid_bdist;
+  const int nfx = int(a.g.nf[0]), nfy = int(a.g.nf[1]);
+  [[maybe_unused]] const i64 cells = a.g.nf[0] * a.g.nf[1];
+  if (lane < count && NNB_CHECK_INDEX(first + lane, M)) {
+    const PointRec<T> rec = a.pts.rec[first + lane];
+    auto& sl = slots[warp][lane];
+    C v{T(0), T(0)};
+    if (NNB_CHECK_INDEX(rec.perm, M)) {
+      v = in[rec.perm];
+      if (a.prephase) v = cmul(v, a.prephase[rec.perm]);
+    }
+    strip_cell<2>(rec, sl.x0, sl.y0);
+    T wt[W];
+    es_weights<W>(rec.frac[0], a.es, a.beta, a.c, wt);
+    const int odd = S::SINGLE ? sl.x0 & 1 : 0;
+    if constexpr (S::SINGLE) sl.kx[0] = sl.kx[S::KXN - 1] = sl.kx[S::KXN - 2] = T(0);
+#pragma unroll
+    for (int i = 0; i < W; ++i) sl.kx[odd + i] = wt[i];
+    es_weights<W>(rec.frac[1], a.es, a.beta, a.c, wt);
+#pragma unroll
+    for (int i = 0; i < W; ++i) sl.ky[i] = wt[i];
+    sl.v = v;
+  }
+  __syncwarp();
+  constexpr int PASSES = (S::ELEMS + 31) / 32;
+  int row[PASSES], col[PASSES];
+#pragma unroll
+  for (int p = 0; p < PASSES; ++p) {
+    row[p] = (lane + 32 * p) / S::PER_ROW;
+    col[p] = (lane + 32 * p) % S::PER_ROW;
+  }
+  for (int j = 0; j < count; ++j) {
+    const auto& pt = slots[warp][j];
+    const C v = pt.v;
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+      if (row[p] >= W) continue;
+      int y = pt.y0 + row[p];
+      if (y >= nfy) y -= nfy;
+      const i64 base = i64(y) * nfx;
+      const T ky = pt.ky[row[p]];
+      if constexpr (S::SINGLE) {
+        const int x = (pt.x0 & ~1) + 2 * col[p];
+        const T k0 = pt.kx[2 * col[p]] * ky, k1 = pt.kx[2 * col[p] + 1] * ky;
+        if (aligned && (pt.x0 & ~1) + 2 * S::PER_ROW <= nfx) {
+          // an even first cell leaves the last pair without weights
+          if (2 * col[p] < W + (pt.x0 & 1) && NNB_CHECK_INDEX(base + x + 1, cells)) {
+            atomic_add_pair(grid + base + x, k0 * v.x, k0 * v.y, k1 * v.x, k1 * v.y);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int off = 2 * col[p] + i - (pt.x0 & 1);  // cell of the footprint
+            int xi = x + i;
+            if (xi >= nfx) xi -= nfx;
+            if (off >= 0 && off < W && NNB_CHECK_INDEX(base + xi, cells)) {
+              const T k = i ? k1 : k0;
+              atomic_add_cplx(grid + base + xi, C{k * v.x, k * v.y});
+            }
+          }
+        }
+      } else {
+        int x = pt.x0 + col[p] / 2;
+        if (x >= nfx) x -= nfx;
+        const T k = pt.kx[col[p] / 2] * ky;
+        if (NNB_CHECK_INDEX(base + x, cells)) {
+          T* cell = reinterpret_cast<T*>(grid + base + x);
+          atomicAdd(cell + (col[p] & 1), k * ((col[p] & 1) ? v.y : v.x));
+        }
+      }
+    }
+  }
+}
+
 template <typename T, int DIM, int W>
 __global__ void __launch_bounds__(kStripInterpThreads)
     interp_strip_kernel(const __grid_constant__ InterpArgs<T> a) {
@@ -320,9 +428,29 @@ u32 strip_chunk(i64 M, int runs_per_warp, int ry) {
   return u32(c < lo ? lo : (c > hi ? hi : c));
 }
 
+// Whether the points of a 2D grid are too sparse for windows: w cells per point or more, at least
+// 6. Uniform points on 4096^2 cells (2048^2 in double precision), windows / direct, in us, at 20,
+// 10 and 5 cells per point: w = 4 133 / 75, 173 / 119, 209 / 223; w = 8 193 / 126, 232 / 212,
+// 344 / 405; double w = 10 138 / 79, 174 / 147, 249 / 290; w = 13 177 / 123, 218 / 239, 303 / 495.
+// The type-3 spread of 5e6 points on 12740^2 cells, w = 6: 2176 / 827 (shared-memory slabs 1335).
+bool sparse_points(const BinGeom& g, i64 M) {
+  return double(M) * std::max(6, g.w) < double(g.nf[0]) * double(g.nf[1]);
+}
+
 template <typename T, int DIM, int W>
 void launch_spread_strip_w(const SpreadArgs<T>& a, cudaStream_t stream) {
   using S = StripShape<T, DIM, W>;
+  if constexpr (DIM == 2) {
+    if (sparse_points(a.g, a.pts.M)) {
+      const i64 ctas = (a.pts.M + 32 * kStripWarps - 1) / (32 * kStripWarps);
+      const bool aligned = a.g.nf[0] % 2 == 0 && a.grid_bdist % 2 == 0 &&
+                           reinterpret_cast<uintptr_t>(a.grid) % 16 == 0;
+      dim3 grid{unsigned(ctas), unsigned(a.batch), 1u};
+      spread_sparse_kernel<T, W><<<grid, 32 * kStripWarps, 0, stream>>>(a, aligned);
+      NNB_LAUNCH_CHECK();
+      return;
+    }
+  }
   const u32 chunk = strip_chunk(a.pts.M, S::NG, S::RY);
   const i64 per_cta = i64(chunk) * S::NG * kStripWarps;
   const i64 ctas = (a.pts.M + per_cta - 1) / per_cta;
