@@ -76,10 +76,17 @@ __device__ __forceinline__ i64 tile_linear_d(const BinGeom& g, const i64 (&t)[3]
   return lin;
 }
 
+// Where the count of bin b lies: eight bins in a row go to eight runs of n8 counts. Atomics on
+// one 32-byte sector of the L2 wait for one another, and clustered points hit neighbouring bins
+// (3e6 points of a Gaussian cluster on 192^3 cells: 303 -> 156 us); the scan reads the eight runs side by
+// side, each coalesced.
+__host__ __device__ __forceinline__ i64 count_slot(i64 b, i64 n8) { return (b & 7) * n8 + (b >> 3); }
+
 template <typename T, int DIM>
 __global__ void __launch_bounds__(kBinBlock)
     bin_count_kernel(BinGeom g, CoordPtrs<T> x, i64 M, u32* counts, u32* ranks, int* err) {
   const i64 stride = i64(gridDim.x) * kBinBlock;
+  const i64 n8 = count_run(g.total_tiles);
   double inv_tile[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) inv_tile[d] = 1.0 / double(g.tile[d]);
@@ -115,8 +122,9 @@ __global__ void __launch_bounds__(kBinBlock)
 #pragma unroll
     for (int u = 0; u < kBinUnroll; ++u) {
       if (base + u * stride < M) {
-        r[u] = NNB_CHECK_INDEX(tile_lin[u], g.total_tiles) ? atomicAdd(&counts[tile_lin[u]], 1u)
-                                                           : 0u;
+        r[u] = NNB_CHECK_INDEX(tile_lin[u], g.total_tiles)
+                   ? atomicAdd(&counts[count_slot(tile_lin[u], n8)], 1u)
+                   : 0u;
       }
     }
 #pragma unroll
@@ -238,14 +246,20 @@ __device__ __forceinline__ u64 block_exclusive_scan(u64 v, u64* total) {
   return res;
 }
 
+// Input item base + k of a scan (base a multiple of kScanItems); n8 > 0: laid out in eight runs
+// (count_slot).
+static_assert(kScanItems == 8, "the scan's threads read one count of each run");
+__device__ __forceinline__ u32 scan_input(const u32* in, i64 base, int k, i64 n, i64 n8) {
+  if (base + k >= n) return 0u;
+  return n8 > 0 ? in[k * n8 + (base >> 3)] : in[base + k];
+}
+
 __global__ void __launch_bounds__(kScanThreads)
-    scan_block_sums_kernel(const u32* in, i64 n, u32* block_sums) {
+    scan_block_sums_kernel(const u32* in, i64 n, i64 n8, u32* block_sums) {
   const i64 base = i64(blockIdx.x) * kScanChunk + threadIdx.x * kScanItems;
   u64 s = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    if (base + k < n) s += in[base + k];
-  }
+  for (int k = 0; k < kScanItems; ++k) s += scan_input(in, base, k, n, n8);
   __shared__ u64 total;
   block_exclusive_scan<kScanThreads>(s, &total);
   if (threadIdx.x == 0) block_sums[blockIdx.x] = u32(total);
@@ -277,13 +291,13 @@ __global__ void __launch_bounds__(kScanThreads) scan_top_kernel(u32* block_sums,
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    scan_apply_kernel(const u32* in, i64 n, const u32* block_offsets, i64 nb, u32* out) {
+    scan_apply_kernel(const u32* in, i64 n, i64 n8, const u32* block_offsets, i64 nb, u32* out) {
   const i64 base = i64(blockIdx.x) * kScanChunk + threadIdx.x * kScanItems;
   u32 v[kScanItems];
   u64 s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = (base + k < n) ? in[base + k] : 0u;
+    v[k] = scan_input(in, base, k, n, n8);
     s += v[k];
   }
   __shared__ u64 total;
@@ -301,7 +315,7 @@ __global__ void __launch_bounds__(kScanThreads)
 constexpr int kScanSmallThreads = 1024;
 constexpr i64 kScanSmall = kScanSmallThreads * kScanItems;
 __global__ void __launch_bounds__(kScanSmallThreads)
-    scan_small_kernel(const u32* in, i64 n, u32* out) {
+    scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out) {
   __shared__ u64 total;
   u64 carry = 0;
   for (i64 off = 0; off < n; off += kScanSmallThreads * kScanItems) {
@@ -310,7 +324,7 @@ __global__ void __launch_bounds__(kScanSmallThreads)
     u64 s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-      v[k] = (base + k < n) ? in[base + k] : 0u;
+      v[k] = scan_input(in, base, k, n, n8);
       s += v[k];
     }
     u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total) + carry;
@@ -354,19 +368,21 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
 
 i64 scan_tmp_words(i64 n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
-void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream) {
+void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
+                           bool runs) {
+  const i64 n8 = runs ? count_run(n) : 0;
   const i64 nb = (n + kScanChunk - 1) / kScanChunk;
   if (nb <= 0) return;
   if (n <= kScanSmall) {
-    scan_small_kernel<<<1, kScanSmallThreads, 0, stream>>>(counts, n, out);
+    scan_small_kernel<<<1, kScanSmallThreads, 0, stream>>>(counts, n, n8, out);
     NNB_LAUNCH_CHECK();
     return;
   }
-  scan_block_sums_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, tmp);
+  scan_block_sums_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, n8, tmp);
   NNB_LAUNCH_CHECK();
   scan_top_kernel<<<1, kScanThreads, 0, stream>>>(tmp, nb);
   NNB_LAUNCH_CHECK();
-  scan_apply_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, tmp, nb, out);
+  scan_apply_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, n8, tmp, nb, out);
   NNB_LAUNCH_CHECK();
 }
 

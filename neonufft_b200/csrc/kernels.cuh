@@ -18,7 +18,10 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
                       int* err_flag, cudaStream_t stream);
 // Exclusive scan of n counts into out[0..n] (out[n] = total). tmp needs scan_tmp_words(n).
 i64 scan_tmp_words(i64 n);
-void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream);
+// runs: the counts lie in eight runs of count_run(n), as launch_bin_count leaves them.
+__host__ __device__ __forceinline__ i64 count_run(i64 n) { return (n + 7) / 8; }
+void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
+                           bool runs = false);
 // Pass 2: one 32-byte record per point (permutation, packed cell, fractions) in tile order.
 template <typename T>
 void launch_perm_checksum(const PointRec<T>* rec, i64 M, unsigned long long* sums,

@@ -341,7 +341,8 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   g_ = g;
   M_ = M;
   const i64 nt = g.total_tiles;
-  counts_.reserve(size_t(nt + 1));  // the error flag behind the counts: one memset for both
+  const i64 nc = 8 * count_run(nt);
+  counts_.reserve(size_t(nc + 1));  // the error flag behind the counts: one memset for both
   bin_start_.reserve(size_t(nt + 1));
   scan_tmp_.reserve(size_t(scan_tmp_words(nt)));
   rec_.reserve(size_t(M));
@@ -352,10 +353,10 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
     work_start_.reserve(size_t(nt + 1));
     work_owner_.reserve(size_t(nt + M / kWorkItemPoints + 2));
   }
-  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nt + 1), stream));
-  int* err = reinterpret_cast<int*>(counts_.data() + nt);
+  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nc + 1), stream));
+  int* err = reinterpret_cast<int*>(counts_.data() + nc);
   launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err, stream);
-  launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream);
+  launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream, true);
   launch_bin_scatter<T>(g, x, M, ranks_.data(), bin_start_.data(), rec_.data(), stream);
   // every z-window transform of these points walks the same list of work items
   if (g.zmajor && M > 0) zwin_build_work_list<T>(g, view(), stream);
