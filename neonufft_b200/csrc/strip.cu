@@ -10,8 +10,9 @@
 // without looking its bin up: both kernels cut the sorted array into equal runs, whatever the
 // distribution of the points, and need no work list.
 //
-// Spreading: a run is walked by RY lanes (RY = 2, 4, 8 or 16 >= W; a warp walks 32 / RY runs side
-// by side). Lane b holds in registers the strip's row y = b (mod RY) of a window of RY rows, P0 =
+// Spreading: a run is walked by RY = W lanes (a warp walks 32 / W runs side by side; with windows
+// rounded up to 8 or 16 rows it walked 4 runs instead of 5 at w = 6, 2 instead of 3 at w = 10).
+// Lane b holds in registers the strip's row y = b (mod RY) of a window of RY rows, P0 =
 // TX + W - 1 cells as pairs of neighbours, and applies each point with packed FMAs: no lane
 // touches another's row, so there are neither atomics nor shared-memory updates per cell. When
 // the next point starts on a later row (or strip) the rows left behind are added to the grid,
@@ -43,8 +44,13 @@ constexpr int kStripInterpThreads = 128;
 
 template <typename T, int DIM, int W>
 struct StripShape {
-  static constexpr int RY = W <= 2 ? 2 : (W <= 4 ? 4 : (W <= 8 ? 8 : 16));  // window rows, lanes per run
-  static constexpr int NG = 32 / RY;                                       // runs per warp
+  static constexpr int RY = W;       // window rows, lanes per run
+  static constexpr int NG = 32 / RY;  // runs per warp
+  // Distance of the row held by lane r of a run from the first row of its window.
+  static __device__ __forceinline__ int offset(int r, int cur) {
+    const int d = r - int(unsigned(cur) % unsigned(RY));
+    return d < 0 ? d + RY : d;
+  }
   static constexpr int TX = DIM == 1 ? 1 : strip_width(sizeof(T), W);
   static constexpr int P0 = DIM == 1 ? 1 : TX + W - 1;  // region cells per row
   static constexpr int NP = (P0 + 1) / 2;               // cell pairs per row
@@ -56,7 +62,7 @@ template <typename T, int DIM, int W>
 struct alignas(16) StripSlotFields {
   using S = StripShape<T, DIM, W>;
   T kx[S::KXN > 0 ? S::KXN : 4];  // over the strip's cells (1D: unused)
-  T ky[S::RY];                    // over the window, zero from W on
+  T ky[S::RY];                    // over the window
   cplx_t<T> v;
   int row, strip;
 };
@@ -98,7 +104,8 @@ __global__ void __launch_bounds__(32 * kStripWarps)
   const i64 first = (i64(blockIdx.x) * kStripWarps + warp) * S::NG * chunk;  // of the warp
   if (first >= M) return;
   const i64 beg = first + i64(grp) * chunk;
-  const int count = int(max(i64(0), min(i64(chunk), M - beg)));
+  // lanes left over by the runs have no points
+  const int count = grp < S::NG ? int(max(i64(0), min(i64(chunk), M - beg))) : 0;
   // run 0 of a warp is its longest
   const int iters = (int(min(i64(chunk), M - first)) + RY - 1) / RY;
 
@@ -200,7 +207,7 @@ __global__ void __launch_bounds__(32 * kStripWarps)
       T wt[W];
       es_weights<W>(rec.frac[DIM - 1], a.es, a.beta, a.c, wt);
 #pragma unroll
-      for (int i = 0; i < RY; ++i) sl.ky[i] = i < W ? wt[i < W ? i : 0] : T(0);
+      for (int i = 0; i < W; ++i) sl.ky[i] = wt[i];
       sl.v = val;
       sl.row = DIM == 2 ? y0 : x0;
       sl.strip = DIM == 2 ? int(unsigned(x0) / unsigned(S::TX)) : 0;
@@ -215,10 +222,9 @@ __global__ void __launch_bounds__(32 * kStripWarps)
         if (dz < (ts == strip ? tp - cur : RY)) flush(i64(cur) + dz);
         cur = tp;
         strip = ts;
-        dz = (rb - cur) & (RY - 1);
+        dz = S::offset(rb, cur);
       }
-      if (RY != W) dirty |= dz < W;
-      else dirty = true;
+      dirty = true;
       const T kw = pt.ky[dz];
       const P wre = Ops::splat(pt.v.x * kw);
       const P wim = Ops::splat(pt.v.y * kw);
