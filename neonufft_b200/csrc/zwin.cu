@@ -295,6 +295,10 @@ template WorkList zwin_work_list<double>(const BinGeom&, const SortedPoints<doub
 
 namespace {
 
+// Window planes per thread (ZShape::PZ).
+template <typename T, int W, int TX, int TY>
+constexpr int zwin_planes = sizeof(T) == 4 && W >= 5 && TX == 4 && TY <= 8 ? 2 : 1;
+
 template <typename T, int W, int TX, int TY>
 void launch_spread_zwin_tw(const SpreadArgs<T>& a, cudaStream_t stream) {
   using S = ZShape<T, W, TX, TY>;
@@ -313,17 +317,23 @@ void launch_spread_zwin_tw(const SpreadArgs<T>& a, cudaStream_t stream) {
     }
   }
   dim3 grid{unsigned(wl.grid), unsigned(a.batch), 1u};
-  spread_zwin_kernel<T, W, TX, TY><<<grid, S::NT, 0, stream>>>(a, ch, wl);
+  if constexpr (zwin_planes<T, W, TX, TY> == 2 && TY == 8) {
+    spread_zwin_planes_kernel<T, W, TX, TY>
+        <<<grid, ZShape<T, W, TX, TY, 2>::NT, 0, stream>>>(a, ch, wl);
+  } else {
+    spread_zwin_kernel<T, W, TX, TY><<<grid, S::NT, 0, stream>>>(a, ch, wl);
+  }
   NNB_LAUNCH_CHECK();
 }
 
 template <typename T, int W, int TX, int TY>
 void launch_interp_zwin_tw(const InterpArgs<T>& a, cudaStream_t stream) {
-  using S = ZShape<T, W, TX, TY>;
   const i64 ncols = i64(a.g.ntiles[0]) * a.g.ntiles[1];
   const ZChunks ch = make_chunks(ncols, a.g.ntiles[2], W);
   const WorkList wl = zwin_work_list(a.g, a.pts, ch);
-  interp_zwin_kernel<T, W, TX, TY><<<unsigned(wl.grid), S::NT, 0, stream>>>(a, ch, wl);
+  constexpr int PZ = zwin_planes<T, W, TX, TY>;
+  interp_zwin_kernel<T, W, TX, TY, PZ>
+      <<<unsigned(wl.grid), ZShape<T, W, TX, TY, PZ>::NT, 0, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
 }
 

@@ -40,17 +40,26 @@ namespace nnb {
 namespace {
 
 // ---- geometry ----------------------------------------------------------------------------------
-template <typename T, int W, int TX, int TY_ = 8>
+// PZ: window planes per thread. With two, a warp holds 8 rows instead of 4, so a point is visited
+// by fewer warps (1.9 of 2 instead of 2.75 of 4 at w = 8, 8-row tiles) and each visit's loads,
+// weights and bookkeeping serve twice the FMAs. 1e7 points on 256^3 cells, w = 8, single precision:
+// spreading 2.03 -> 1.86 ms, interpolation 2.58 -> 2.43 ms (with one plane the polynomial weights
+// had already taken interpolation from 2.73 to 2.58 ms). Spreading on 4-row tiles keeps one plane
+// (1e8 points on 480^3 cells: 16.5 against 18.2 ms with two), and so does double precision (3e6
+// clustered points, w = 7: spreading 1.19 against 1.26 ms, interpolation 1.30 against 1.29).
+template <typename T, int W, int TX, int TY_ = 8, int PZ_ = 1>
 struct ZShape {
+  static constexpr int PZ = PZ_;
   static constexpr bool WIDE = W > 8;
   // Window planes = z residues (>= W). Wide kernels take exactly W: rounded up to 16, half of the
   // FMAs of w = 10 would be on planes outside the footprint.
   static constexpr int RZ = W <= 4 ? 4 : (W <= 8 ? 8 : W);
-  static constexpr int LA = 32 / RZ;                // rows per warp
+  static constexpr int ZL = RZ / PZ;                // lanes along z
+  static constexpr int LA = 32 / ZL;                // rows per warp
   static constexpr int TY = TY_;                    // tile y (4, 8 or 16)
   static constexpr int P1 = TY + W - 1;             // region y extent
   // region rows (>= P1, a multiple of the rows per warp)
-  static constexpr int RY = TY == 4 || WIDE ? (P1 + LA - 1) / LA * LA : TY + 8;
+  static constexpr int RY = TY == 4 || WIDE || PZ > 1 ? (P1 + LA - 1) / LA * LA : TY + 8;
   static constexpr int NWARP = RY / LA;
   static constexpr int NT = 32 * NWARP;             // threads per CTA
   static constexpr int P0 = TX + W - 1;             // region x extent (cells)
@@ -60,19 +69,26 @@ struct ZShape {
   static constexpr int RZS = (RZ + 3) / 4 * 4;      // staged kz values (16-byte multiple)
   // points staged at a time, each warp its share
   static constexpr int BATCH =
-      sizeof(T) == 4 && !WIDE ? (NWARP == 1 ? 32 : (NWARP % 3 == 0 ? 48 : 64)) : 32;
+      sizeof(T) == 4 && !WIDE && PZ == 1 ? (NWARP == 1 ? 32 : (NWARP % 3 == 0 ? 48 : 64)) : 32;
   static constexpr int PW = (BATCH + NWARP - 1) / NWARP;  // points staged per warp
   static constexpr int G = WIDE ? 4 : 8;            // points reduced together (interpolation)
   // CTAs per SM the interpolation kernel is compiled for: 6 in single precision (78 registers,
   // no spills; 86 uncapped, which allows only 5 CTAs and measured 6 % slower), 5 in double.
-  // The wide kernels have a budget of 128 registers.
-  static constexpr int WIDE_CTAS = 65536 / (NT * 128) > 0 ? 65536 / (NT * 128) : 1;
-  static constexpr int INTERP_CTAS = WIDE ? WIDE_CTAS : (sizeof(T) == 4 ? 6 : 5);
+  // Two planes per thread: 96 registers (interpolation), 92 (spreading).
+  static constexpr int PZ_INTERP_CTAS = 65536 / (NT * 96);
+  static constexpr int SPREAD_CTAS = 65536 / (NT * 92);
+  // The wide kernels have a budget of 112 registers (3 CTAs of 192 threads at w = 10 in double
+  // precision, a few spills; uncapped, ptxas takes 157 and 2 CTAs fit: spreading 5e5 points
+  // 512 -> 475 us, interpolation 628 -> 568 us).
+  static constexpr int WIDE_CTAS = 65536 / (NT * 112) > 0 ? 65536 / (NT * 112) : 1;
+  static constexpr int INTERP_CTAS =
+      WIDE ? WIDE_CTAS : (PZ > 1 ? PZ_INTERP_CTAS : (sizeof(T) == 4 ? 6 : 5));
   // CTAs per SM the two-vector spreading kernel is compiled for: a budget of about 88 registers
   // a thread (7 CTAs of 96 threads; ptxas then allocates 80 registers and spills 24 bytes for
   // w = 8). Uncapped, the allocator takes 158 registers for w = 8, which leaves 2 CTAs per SM.
   static constexpr int SPREAD2_CTAS = 65536 / (NT * 88) > 0 ? 65536 / (NT * 88) : 1;
   static_assert(W <= RZ && P1 <= RY, "window smaller than the kernel footprint");
+  static_assert(RZ % PZ == 0 && (PZ == 1 || !WIDE), "planes per thread");
   static_assert(PW <= 32 && BATCH % G == 0, "staging threads");
   // Residue of a plane (>= 0), and its distance from residue r of a window starting at cur.
   static __device__ __forceinline__ int offset(int r, int cur) {
@@ -90,9 +106,9 @@ template <typename T>
 constexpr int kInterpFusedCtas = sizeof(T) == 4 ? 6 : 4;
 
 // Per-point data staged in shared memory (one slot per point of a batch).
-template <typename T, int W, int TX, int TY = 8>
+template <typename T, int W, int TX, int TY = 8, int PZ = 1>
 struct alignas(16) ZSlotFields {
-  using S = ZShape<T, W, TX, TY>;
+  using S = ZShape<T, W, TX, TY, PZ>;
   T kx[S::KXN];    // kx over the region's x range, zero outside the footprint
   T ky[S::RYS];    // ky over the region rows, zero outside the footprint
   T kz[S::RZS];    // kz per window offset, zero beyond w
@@ -108,9 +124,10 @@ struct ZSlotPad {
 };
 template <>
 struct ZSlotPad<true> {};
-template <typename T, int W, int TX, int TY = 8>
+template <typename T, int W, int TX, int TY = 8, int PZ = 1>
 struct alignas(16) ZSlot
-    : ZSlotFields<T, W, TX, TY>, ZSlotPad<(sizeof(ZSlotFields<T, W, TX, TY>) / 16) % 2 == 1> {};
+    : ZSlotFields<T, W, TX, TY, PZ>,
+      ZSlotPad<(sizeof(ZSlotFields<T, W, TX, TY, PZ>) / 16) % 2 == 1> {};
 
 // Stages `count` (<= 16) bin-sorted records `recs` into slots[0 .. count), one warp: lanes
 // 0 .. count - 1 load the records (and, for spreading, the strengths; with `v2_out`, also the
@@ -123,13 +140,13 @@ struct alignas(16) ZSlot
 // POLY: kernel values by the polynomials of the pieces; double precision gives each lane of the
 // pair its half of kz (single precision measured slower that way: 1.98 against 1.86 ms per 1e7
 // points) while both evaluate all of kz in single.
-template <typename T, int W, int TX, bool SPREAD, int TY = 8, bool POLY = true>
-__device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const PointRec<T>* recs,
+template <typename T, int W, int TX, bool SPREAD, int TY = 8, int PZ = 1, bool POLY = true>
+__device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY, PZ>* slots, const PointRec<T>* recs,
                                            int count, const cplx_t<T>* in,
                                            const cplx_t<T>* prephase,
                                            const EsPoly<T>& es, T beta, T c, int lane, i64 num, const cplx_t<T>* in2 = nullptr,
                                            cplx_t<T>* v2_out = nullptr) {
-  using S = ZShape<T, W, TX, TY>;
+  using S = ZShape<T, W, TX, TY, PZ>;
   using C = cplx_t<T>;
   constexpr unsigned kFull = 0xffffffffu;
   PointRec<T> rec;
@@ -162,7 +179,7 @@ __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const Poi
   const T fz = __shfl_sync(kFull, rec.frac[2], p);
   const T vx = __shfl_sync(kFull, v.x, p);
   const T vy = __shfl_sync(kFull, v.y, p);
-  ZSlot<T, W, TX, TY>& sl = slots[p < count ? p : 0];
+  ZSlot<T, W, TX, TY, PZ>& sl = slots[p < count ? p : 0];
   constexpr int kZero16 = int((S::KXN + S::RYS) * sizeof(T) / 16);  // kx and ky are contiguous
   constexpr int kHalf = (kZero16 + 1) / 2;
   if (p < count) {
@@ -177,16 +194,7 @@ __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const Poi
     const int lx = int(loc & 0xFu);
     const int ly = int((loc >> 4) & 0xFu);
     T* dst = h ? sl.ky + ly : sl.kx + lx;
-    if constexpr (!POLY) {
-      const T f = h ? fy : fx;
-#pragma unroll
-      for (int k = 0; k < W; ++k) dst[k] = es_eval_fast<T>(f + T(k), beta, c);
-#pragma unroll
-      for (int i = 0; i < S::RZS / 2; ++i) {
-        const int k = h * (S::RZS / 2) + i;
-        sl.kz[k] = k < W ? es_eval_fast<T>(fz + T(k), beta, c) : T(0);
-      }
-    } else {
+    if constexpr (POLY) {
       T wt[W];
       es_weights<W>(h ? fy : fx, es, beta, c, wt);
 #pragma unroll
@@ -206,6 +214,15 @@ __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY>* slots, const Poi
           const T hi = H + i < W ? wt[H + i < W ? H + i : 0] : T(0);
           sl.kz[h * H + i] = h ? hi : lo;
         }
+      }
+    } else {
+      const T f = h ? fy : fx;
+#pragma unroll
+      for (int k = 0; k < W; ++k) dst[k] = es_eval_fast<T>(f + T(k), beta, c);
+#pragma unroll
+      for (int i = 0; i < S::RZS / 2; ++i) {
+        const int k = h * (S::RZS / 2) + i;
+        sl.kz[k] = k < W ? es_eval_fast<T>(fz + T(k), beta, c) : T(0);
       }
     }
     if (h == 0) {
@@ -264,9 +281,9 @@ __device__ __forceinline__ bool zcta(const BinGeom& g, const u32* bin_start, ZCh
 }
 
 // Thread layout shared by both kernels.
-template <typename T, int W, int TX, int TY = 8>
+template <typename T, int W, int TX, int TY = 8, int PZ = 1>
 struct ZThread {
-  using S = ZShape<T, W, TX, TY>;
+  using S = ZShape<T, W, TX, TY, PZ>;
   int tid, warp, lane, ra, rb, a_lo;
   bool active;  // the lane holds a row (with LA RZ < 32 lanes per warp, some do not)
   int stage_j;  // batch slot this thread stages (< BATCH), or -1
@@ -274,9 +291,9 @@ struct ZThread {
     tid = threadIdx.x;
     warp = tid >> 5;
     lane = tid & 31;
-    active = S::LA * S::RZ == 32 || lane < S::LA * S::RZ;
+    active = S::LA * S::ZL == 32 || lane < S::LA * S::ZL;
     ra = warp * S::LA + lane % S::LA;  // region row
-    rb = active ? lane / S::LA : 0;     // z residue
+    rb = active ? lane / S::LA : 0;     // z residue of the first plane, the next ZL further on
     a_lo = warp * S::LA;                // first row of this warp
     // consecutive lanes stage consecutive slots (the slot stride is 4 words times an odd
     // number, so their shared-memory stores fall in different banks)
@@ -288,10 +305,10 @@ struct ZThread {
 
 // ---- spreading ---------------------------------------------------------------------------------
 // NV strength vectors on the same points (NV = 2: the second vector's staged strengths).
-template <typename T, int W, int TX, int TY = 8, int NV = 1>
+template <typename T, int W, int TX, int TY = 8, int NV = 1, int PZ = 1>
 struct ZSpreadShared {
-  ZSlot<T, W, TX, TY> slots[2][ZShape<T, W, TX, TY>::BATCH];
-  cplx_t<T> v2[2][NV > 1 ? ZShape<T, W, TX, TY>::BATCH : 1];
+  ZSlot<T, W, TX, TY, PZ> slots[2][ZShape<T, W, TX, TY, PZ>::BATCH];
+  cplx_t<T> v2[2][NV > 1 ? ZShape<T, W, TX, TY, PZ>::BATCH : 1];
 };
 
 // Spreads work item `item` of batch entries batch .. batch + NV - 1 (one CTA; every thread
@@ -299,22 +316,23 @@ struct ZSpreadShared {
 // serve two strength vectors on the same points (type-3 batches, repeated type-1 transforms):
 // the second vector's row sums sit in their own registers and go to the next grid (at
 // grid_bdist); a missing second entry (an odd batch) is skipped.
-template <typename T, int W, int TX, int TY = 8, int NV = 1>
+template <typename T, int W, int TX, int TY = 8, int NV = 1, int PZ = 1>
 __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks ch,
                                                  const WorkList& wl, u32 item, int batch,
-                                                 ZSpreadShared<T, W, TX, TY, NV>& sh) {
+                                                 ZSpreadShared<T, W, TX, TY, NV, PZ>& sh) {
   static_assert(NV == 1 || NV == 2, "one or two strength vectors per pass");
-  using S = ZShape<T, W, TX, TY>;
+  static_assert(NV == 1 || PZ == 1, "two vectors use one plane per thread");
+  using S = ZShape<T, W, TX, TY, PZ>;
   using Ops = Packed<T>;
   using P = typename Ops::P;
   using C = cplx_t<T>;
-  using Slot = ZSlot<T, W, TX, TY>;
+  using Slot = ZSlot<T, W, TX, TY, PZ>;
   auto& slots = sh.slots;
 
   const BinGeom& g = a.g;
   ZCta cta;
   if (!zcta(g, a.pts.bin_start, ch, wl, item, cta)) return;
-  const ZThread<T, W, TX, TY> th;
+  const ZThread<T, W, TX, TY, PZ> th;
   const C* in = a.in + batch * a.in_bdist;
   C* grid = a.grid + batch * a.grid_bdist;
   const bool has2 = NV > 1 && batch + 1 < a.batch;  // the second vector exists
@@ -325,26 +343,30 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
   const i64 row_y = has_row ? wrap_add(i64(cta.ty) * S::TY, th.ra, nfy) : 0;
   const i64 gx0 = i64(cta.tx) * TX;
 
-  // real / imaginary parts of cell pairs (2q, 2q + 1) of the row, per strength vector
-  P are[NV][S::NP], aim[NV][S::NP];
+  // real / imaginary parts of cell pairs (2q, 2q + 1) of the row, per strength vector or plane
+  constexpr int NA = NV * PZ;
+  P are[NA][S::NP], aim[NA][S::NP];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
+  for (int v = 0; v < NA; ++v) {
 #pragma unroll
     for (int q = 0; q < S::NP; ++q) are[v][q] = aim[v][q] = Ops::zero();
   }
   bool dirty = false;
 
-  // Adds this thread's row of plane p (absolute; may exceed nfz) to the grid(s) and clears it.
+  // Adds this thread's row of plane p (absolute; may exceed nfz; the thread's z-th plane, a
+  // constant) to the grid(s) and clears it.
   // The region's x range lies inside the grid and its rows start 16-byte aligned (the usual
   // case): whole cell pairs are added with one vector atomic each.
   const bool pairs = !narrow && gx0 + S::P0 <= nfx && (nfx % 2) == 0 &&
                      (reinterpret_cast<size_t>(grid) % 16) == 0 &&
                      (NV == 1 || (a.grid_bdist % 2) == 0);
-  auto flush = [&](int p) {
+  auto flush = [&](auto zc, int p) {
+    constexpr int z = decltype(zc)::value;
     if (has_row && dirty) {
       const i64 base = (wrap_plane(p, nfz) * nfy + row_y) * nfx;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
+        const int k = v + z;
         if (v == 1 && !has2) break;
         C* row = grid + v * a.grid_bdist + base;
         if (pairs) {
@@ -353,11 +375,11 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
           for (int q = 0; q < S::NP; ++q) {
             if (2 * q + 1 < S::P0) {
               if (NNB_CHECK_INDEX(base + gx0 + 2 * q + 1, cells)) {
-                atomic_add_pair(r + 2 * q, Ops::lo(are[v][q]), Ops::lo(aim[v][q]),
-                                Ops::hi(are[v][q]), Ops::hi(aim[v][q]));
+                atomic_add_pair(r + 2 * q, Ops::lo(are[k][q]), Ops::lo(aim[k][q]),
+                                Ops::hi(are[k][q]), Ops::hi(aim[k][q]));
               }
             } else if (NNB_CHECK_INDEX(base + gx0 + 2 * q, cells)) {
-              atomic_add_cplx(r + 2 * q, C{Ops::lo(are[v][q]), Ops::lo(aim[v][q])});
+              atomic_add_cplx(r + 2 * q, C{Ops::lo(are[k][q]), Ops::lo(aim[k][q])});
             }
           }
         } else {
@@ -365,11 +387,11 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
           for (int q = 0; q < S::NP; ++q) {
             const i64 x0 = wrap_x(gx0, 2 * q, nfx, narrow);
             if (NNB_CHECK_INDEX(base + x0, cells)) {
-              atomic_add_cplx(&row[x0], C{Ops::lo(are[v][q]), Ops::lo(aim[v][q])});
+              atomic_add_cplx(&row[x0], C{Ops::lo(are[k][q]), Ops::lo(aim[k][q])});
             }
             const i64 x1 = wrap_x(gx0, 2 * q + 1, nfx, narrow);
             if (2 * q + 1 < S::P0 && NNB_CHECK_INDEX(base + x1, cells)) {
-              atomic_add_cplx(&row[x1], C{Ops::hi(are[v][q]), Ops::hi(aim[v][q])});
+              atomic_add_cplx(&row[x1], C{Ops::hi(are[k][q]), Ops::hi(aim[k][q])});
             }
           }
         }
@@ -377,15 +399,18 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
 #pragma unroll
-        for (int q = 0; q < S::NP; ++q) are[v][q] = aim[v][q] = Ops::zero();
+        for (int q = 0; q < S::NP; ++q) are[v + z][q] = aim[v + z][q] = Ops::zero();
       }
     }
-    dirty = false;
+    if (PZ == 1) dirty = false;
   };
+  using Z0 = std::integral_constant<int, 0>;
+  using Z1 = std::integral_constant<int, PZ - 1>;
 
-  // One vector in single precision keeps the formula: with the polynomials ptxas takes 96 instead
-  // of 55 registers and 1e8 points on 480^3 cells 23.5 instead of 16.5 ms (20.2 capped at 64).
-  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || NV > 1;
+  // One vector and one plane per thread in single precision keeps the formula: with the
+  // polynomials ptxas takes 96 instead of 55 registers and 1e8 points on 480^3 cells 23.5 instead
+  // of 16.5 ms (20.2 capped at 64). With two planes they take 1e7 points from 2.32 to 1.86 ms.
+  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || NV > 1 || PZ > 1;
   const u32 npts = cta.pend - cta.pbeg;
   const int nbatch = int((npts + S::BATCH - 1) / S::BATCH);
   auto stage = [&](int k) {
@@ -399,7 +424,7 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
         break;
       }
       // NV = 2: the second vector's strengths at the same points (zeros when it is missing)
-      stage_warp<T, W, TX, true, TY, kPoly>(slots[k & 1] + th.warp * PW + c0,
+      stage_warp<T, W, TX, true, TY, PZ, kPoly>(slots[k & 1] + th.warp * PW + c0,
                                  a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
                                  min(count - c0, 16), in, a.prephase, a.es, a.beta, a.c, th.lane,
                                  a.pts.M, NV > 1 && has2 ? in + a.in_bdist : nullptr,
@@ -432,22 +457,28 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
           const int tp = sl.lyp >> 4;
           if (tp != cur) {  // advance the window: planes [cur, tp) are complete
             if constexpr (S::WIDE) {
-              if (dz < tp - cur) flush(cur + dz);
-            } else {
-              // (flushing by dz < tp - cur here costs the narrow kernels 6 %)
+              if (dz < tp - cur) flush(Z0{}, cur + dz);
+            } else {  // (by dz < tp - cur as above: 4 % slower)
               const int n = min(tp - cur, S::RZ);
               for (int i = 0; i < n; ++i) {
-                if (th.rb == ((cur + i) & (S::RZ - 1))) flush(cur + i);
+                const int r = (cur + i) & (S::RZ - 1);
+                if (th.rb == r) flush(Z0{}, cur + i);
+                if (PZ > 1 && th.rb + S::ZL == r) flush(Z1{}, cur + i);
               }
             }
             cur = tp;
             dz = S::offset(th.rb, cur);
           }
           dirty = true;
-          const T kw = sl.ky[th.ra] * sl.kz[dz];
+          const T ky = sl.ky[th.ra];
           const C v = sl.v;
-          const P wre = Ops::splat(v.x * kw);
-          const P wim = Ops::splat(v.y * kw);
+          P wre[PZ], wim[PZ];
+#pragma unroll
+          for (int z = 0; z < PZ; ++z) {  // planes rb and rb + ZL = RZ / 2: offsets dz, dz ^ ZL
+            const T kw = ky * sl.kz[z ? dz ^ S::ZL : dz];
+            wre[z] = Ops::splat(v.x * kw);
+            wim[z] = Ops::splat(v.y * kw);
+          }
 #pragma unroll
           for (int q = 0; q < S::NP; q += 2) {
             P kk[2];
@@ -455,8 +486,11 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
               if (q + u < S::NP) {
-                are[0][q + u] = Ops::fma(kk[u], wre, are[0][q + u]);
-                aim[0][q + u] = Ops::fma(kk[u], wim, aim[0][q + u]);
+#pragma unroll
+                for (int z = 0; z < PZ; ++z) {
+                  are[z][q + u] = Ops::fma(kk[u], wre[z], are[z][q + u]);
+                  aim[z][q + u] = Ops::fma(kk[u], wim[z], aim[z][q + u]);
+                }
               }
             }
           }
@@ -486,12 +520,13 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
           m &= ~run;
           if (tp != cur) {  // advance the window: planes [cur, tp) are complete
             if constexpr (S::WIDE) {
-              if (dz < tp - cur) flush(cur + dz);
-            } else {
-              // (flushing by dz < tp - cur here costs the narrow kernels 6 %)
+              if (dz < tp - cur) flush(Z0{}, cur + dz);
+            } else {  // (by dz < tp - cur as above: 4 % slower)
               const int n = min(tp - cur, S::RZ);
               for (int i = 0; i < n; ++i) {
-                if (th.rb == ((cur + i) & (S::RZ - 1))) flush(cur + i);
+                const int r = (cur + i) & (S::RZ - 1);
+                if (th.rb == r) flush(Z0{}, cur + i);
+                if (PZ > 1 && th.rb + S::ZL == r) flush(Z1{}, cur + i);
               }
             }
             cur = tp;
@@ -533,7 +568,8 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
     if (k + 1 < nbatch) stage(k + 1);
     __syncthreads();
   }
-  flush(cur + dz);  // the rest of the window
+  flush(Z0{}, cur + dz);  // the rest of the window
+  if (PZ > 1) flush(Z1{}, cur + (dz ^ S::ZL));
 }
 
 // Double precision is held to 100 registers (5 CTAs of 128 threads): uncapped, ptxas takes 106
@@ -547,6 +583,25 @@ __global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT,
   spread_zwin_item<T, W, TX, TY>(a, ch, wl, blockIdx.x, int(blockIdx.y), sh);
 }
 
+// Kernel widths above 8.
+template <typename T, int W, int TX, int TY>
+__global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT, ZShape<T, W, TX, TY>::WIDE_CTAS)
+    spread_zwin_wide_kernel(const __grid_constant__ SpreadArgs<T> a, ZChunks ch,
+                            const __grid_constant__ WorkList wl) {
+  __shared__ ZSpreadShared<T, W, TX, TY> sh;
+  spread_zwin_item<T, W, TX, TY>(a, ch, wl, blockIdx.x, int(blockIdx.y), sh);
+}
+
+// Two planes per thread.
+template <typename T, int W, int TX, int TY>
+__global__ void __launch_bounds__(ZShape<T, W, TX, TY, 2>::NT,
+                                  ZShape<T, W, TX, TY, 2>::SPREAD_CTAS)
+    spread_zwin_planes_kernel(const __grid_constant__ SpreadArgs<T> a, ZChunks ch,
+                              const __grid_constant__ WorkList wl) {
+  __shared__ ZSpreadShared<T, W, TX, TY, 1, 2> sh;
+  spread_zwin_item<T, W, TX, TY, 1, 2>(a, ch, wl, blockIdx.x, int(blockIdx.y), sh);
+}
+
 // Two strength vectors per CTA: batch entries 2 blockIdx.y and 2 blockIdx.y + 1.
 template <typename T, int W, int TX, int TY>
 __global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT, ZShape<T, W, TX, TY>::SPREAD2_CTAS)
@@ -557,25 +612,25 @@ __global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT, ZShape<T, W, TX, TY>
 }
 
 // ---- interpolation -----------------------------------------------------------------------------
-template <typename T, int W, int TX, int TY = 8>
+template <typename T, int W, int TX, int TY = 8, int PZ = 1>
 struct ZInterpShared {
-  using S = ZShape<T, W, TX, TY>;
+  using S = ZShape<T, W, TX, TY, PZ>;
   static constexpr int RS = 33;  // odd row stride of the transpose buffer: conflict-free reads
-  ZSlot<T, W, TX, TY> slots[2][S::BATCH];
+  ZSlot<T, W, TX, TY, PZ> slots[2][S::BATCH];
   cplx_t<T> red[S::NWARP][S::G][RS];
   cplx_t<T> res[2][S::NWARP][S::BATCH];
 };
 
 // Interpolates work item `item` (one CTA; every thread calls it).
-template <typename T, int W, int TX, int TY = 8>
+template <typename T, int W, int TX, int TY = 8, int PZ = 1>
 __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks ch,
                                                  const WorkList& wl, u32 item,
-                                                 ZInterpShared<T, W, TX, TY>& sh) {
-  using S = ZShape<T, W, TX, TY>;
+                                                 ZInterpShared<T, W, TX, TY, PZ>& sh) {
+  using S = ZShape<T, W, TX, TY, PZ>;
   using Ops = Packed<T>;
   using P = typename Ops::P;
   using C = cplx_t<T>;
-  using Slot = ZSlot<T, W, TX, TY>;
+  using Slot = ZSlot<T, W, TX, TY, PZ>;
   constexpr int G = S::G;
   auto& slots = sh.slots;
   auto& red = sh.red;
@@ -584,7 +639,7 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
   const BinGeom& g = a.g;
   ZCta cta;
   if (!zcta(g, a.pts.bin_start, ch, wl, item, cta)) return;
-  const ZThread<T, W, TX, TY> th;
+  const ZThread<T, W, TX, TY, PZ> th;
   const C* grid = a.grid;
   const i64 nfx = g.nf[0], nfy = g.nf[1], nfz = g.nf[2];
   [[maybe_unused]] const i64 cells = nfx * nfy * nfz;
@@ -595,15 +650,19 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
 
   // Row values of the window plane: real / imaginary parts of cell pairs (2q, 2q + 1); rows
   // outside the region stay zero.
-  P gre[S::NP], gim[S::NP];
+  P gre[PZ][S::NP], gim[PZ][S::NP];
 #pragma unroll
-  for (int q = 0; q < S::NP; ++q) gre[q] = gim[q] = Ops::zero();
+  for (int z = 0; z < PZ; ++z) {
+#pragma unroll
+    for (int q = 0; q < S::NP; ++q) gre[z][q] = gim[z][q] = Ops::zero();
+  }
   // The region's x range lies inside the grid (the usual case): contiguous row segments.
   const bool contiguous = !narrow && gx0 + S::P0 <= nfx;
   // ... and its cell pairs start 16-byte aligned (single precision): one 16-byte load per pair
   const bool pairs16 = sizeof(T) == 4 && contiguous && (nfx % 2) == 0 &&
                        (reinterpret_cast<size_t>(grid) % 16) == 0;
-  auto load_row = [&](int p) {
+  auto load_row = [&](auto zc, int p) {
+    constexpr int z = decltype(zc)::value;
     if (!has_row) return;
     const i64 base = (wrap_plane(p, nfz) * nfy + row_y) * nfx;
     const C* row = grid + base;
@@ -616,13 +675,13 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
             if (NNB_CHECK_INDEX(base + gx0 + 2 * q + 1, cells)) {
               v = *reinterpret_cast<const float4*>(row + gx0 + 2 * q);
             }
-            gre[q] = Ops::pack(v.x, v.z);
-            gim[q] = Ops::pack(v.y, v.w);
+            gre[z][q] = Ops::pack(v.x, v.z);
+            gim[z][q] = Ops::pack(v.y, v.w);
           } else {
             C c0{T(0), T(0)};
             if (NNB_CHECK_INDEX(base + gx0 + 2 * q, cells)) c0 = row[gx0 + 2 * q];
-            gre[q] = Ops::pack(c0.x, T(0));
-            gim[q] = Ops::pack(c0.y, T(0));
+            gre[z][q] = Ops::pack(c0.x, T(0));
+            gim[z][q] = Ops::pack(c0.y, T(0));
           }
         }
         return;
@@ -635,8 +694,8 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
       const i64 x1 = contiguous ? gx0 + 2 * q + 1 : wrap_x(gx0, 2 * q + 1, nfx, narrow);
       if (NNB_CHECK_INDEX(base + x0, cells)) c0 = row[x0];
       if (2 * q + 1 < S::P0 && NNB_CHECK_INDEX(base + x1, cells)) c1 = row[x1];
-      gre[q] = Ops::pack(c0.x, c1.x);
-      gim[q] = Ops::pack(c0.y, c1.y);
+      gre[z][q] = Ops::pack(c0.x, c1.x);
+      gim[z][q] = Ops::pack(c0.y, c1.y);
     }
   };
   const u32 npts = cta.pend - cta.pbeg;
@@ -651,7 +710,7 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
                            a.pts.M)) {
         break;
       }
-      stage_warp<T, W, TX, false, TY>(slots[k & 1] + th.warp * PW + c0,
+      stage_warp<T, W, TX, false, TY, PZ>(slots[k & 1] + th.warp * PW + c0,
                                   a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
                                   min(count - c0, 16), nullptr, nullptr, a.es, a.beta, a.c, th.lane,
                                   a.pts.M);
@@ -681,7 +740,10 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
   __syncthreads();
   int cur = slots[0][0].lyp >> 4;  // window start: the first point's plane
   int dz = S::offset(th.rb, cur);
-  load_row(cur + dz);
+  using Z0 = std::integral_constant<int, 0>;
+  using Z1 = std::integral_constant<int, PZ - 1>;
+  load_row(Z0{}, cur + dz);
+  if (PZ > 1) load_row(Z1{}, cur + (dz ^ S::ZL));
 
   for (int k = 0; k < nbatch; ++k) {
     const int nb = int(min(npts - u32(k) * S::BATCH, u32(S::BATCH)));
@@ -696,22 +758,36 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
     }
     // Row sum of an owned point over this thread's row, times ky kz.
     auto partial = [&](const Slot& sl) -> C {
-      const T kw = sl.ky[th.ra] * sl.kz[dz];
-      P sr0 = Ops::zero(), sr1 = Ops::zero(), si0 = Ops::zero(), si1 = Ops::zero();
+      // one plane: two chains, over the even and the odd pairs; two planes: a chain each
+      P sr[2], si[2];
+      sr[0] = sr[1] = si[0] = si[1] = Ops::zero();
 #pragma unroll
       for (int q = 0; q < S::NP; q += 2) {
         P kp[2];
         load_pairs<T>(&sl.kx[2 * q], kp);
-        sr0 = Ops::fma(kp[0], gre[q], sr0);
-        si0 = Ops::fma(kp[0], gim[q], si0);
-        if (q + 1 < S::NP) {
-          sr1 = Ops::fma(kp[1], gre[q + 1], sr1);
-          si1 = Ops::fma(kp[1], gim[q + 1], si1);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (q + u >= S::NP) continue;
+#pragma unroll
+          for (int z = 0; z < PZ; ++z) {
+            const int k = PZ > 1 ? z : u;
+            sr[k] = Ops::fma(kp[u], gre[z][q + u], sr[k]);
+            si[k] = Ops::fma(kp[u], gim[z][q + u], si[k]);
+          }
         }
       }
-      const P sr = Ops::add(sr0, sr1);
-      const P si = Ops::add(si0, si1);
-      return C{kw * (Ops::lo(sr) + Ops::hi(sr)), kw * (Ops::lo(si) + Ops::hi(si))};
+      const T ky = sl.ky[th.ra];
+      if constexpr (PZ > 1) {
+        const P k0 = Ops::splat(sl.kz[dz]), k1 = Ops::splat(sl.kz[dz ^ S::ZL]);
+        const P r = Ops::fma(k0, sr[0], Ops::fma(k1, sr[1], Ops::zero()));
+        const P i = Ops::fma(k0, si[0], Ops::fma(k1, si[1], Ops::zero()));
+        return C{ky * (Ops::lo(r) + Ops::hi(r)), ky * (Ops::lo(i) + Ops::hi(i))};
+      } else {
+        const T kw = ky * sl.kz[dz];
+        const P r = Ops::add(sr[0], sr[1]);
+        const P i = Ops::add(si[0], si[1]);
+        return C{kw * (Ops::lo(r) + Ops::hi(r)), kw * (Ops::lo(i) + Ops::hi(i))};
+      }
     };
     for (int j0 = 0; j0 < nb; j0 += G) {
       // Points are plane-sorted: if the group's last point is on the window's first plane, so
@@ -734,11 +810,17 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
             const int lyp = sl.lyp;
             const int tp = lyp >> 4;
             if (tp != cur) {  // advance the window: rows of planes [cur, tp) move on by RZ
-              if (S::WIDE || tp - cur >= S::RZ) {
-                if (dz < tp - cur) load_row(tp + S::offset(th.rb, tp));
+              if constexpr (S::WIDE) {
+                if (dz < tp - cur) load_row(Z0{}, tp + S::offset(th.rb, tp));
+              } else if (tp - cur >= S::RZ) {
+                const int nz = S::offset(th.rb, tp);
+                load_row(Z0{}, tp + nz);
+                if (PZ > 1) load_row(Z1{}, tp + (nz ^ S::ZL));
               } else {
                 for (int i = 0; i < tp - cur; ++i) {
-                  if (th.rb == ((cur + i) & (S::RZ - 1))) load_row(cur + i + S::RZ);
+                  const int r = (cur + i) & (S::RZ - 1);
+                  if (th.rb == r) load_row(Z0{}, cur + i + S::RZ);
+                  if (PZ > 1 && th.rb + S::ZL == r) load_row(Z1{}, cur + i + S::RZ);
                 }
               }
               cur = tp;
@@ -777,8 +859,9 @@ __device__ __forceinline__ void interp_zwin_item(const InterpArgs<T>& a, ZChunks
   output(nbatch - 1);
 }
 
-template <typename T, int W, int TX, int TY>
-__global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT, ZShape<T, W, TX, TY>::INTERP_CTAS)
+template <typename T, int W, int TX, int TY, int PZ = 1>
+__global__ void __launch_bounds__(ZShape<T, W, TX, TY, PZ>::NT,
+                                  ZShape<T, W, TX, TY, PZ>::INTERP_CTAS)
     interp_zwin_kernel(const __grid_constant__ InterpArgs<T> a, ZChunks ch,
                        const __grid_constant__ WorkList wl) {
   if constexpr (ZShape<T, W, TX, TY>::WIDE) {  // more than the 48 KB of static shared memory
@@ -786,8 +869,8 @@ __global__ void __launch_bounds__(ZShape<T, W, TX, TY>::NT, ZShape<T, W, TX, TY>
     interp_zwin_item<T, W, TX, TY>(a, ch, wl, blockIdx.x,
                                    *reinterpret_cast<ZInterpShared<T, W, TX, TY>*>(smem_raw));
   } else {
-    __shared__ ZInterpShared<T, W, TX, TY> sh;
-    interp_zwin_item<T, W, TX, TY>(a, ch, wl, blockIdx.x, sh);
+    __shared__ ZInterpShared<T, W, TX, TY, PZ> sh;
+    interp_zwin_item<T, W, TX, TY, PZ>(a, ch, wl, blockIdx.x, sh);
   }
 }
 

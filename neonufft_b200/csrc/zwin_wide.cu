@@ -3,7 +3,7 @@
 //
 // The shared-memory slabs that took these widths (spread.cu, interp.cu) are bound by the chain of
 // shared-memory accesses from point to point: 5e5 points on 128 x 120 x 128 cells, w = 10, double
-// precision, spread in 2.87 ms and interpolated in 1.56 ms; here 0.62 and 0.79 ms, bound by the
+// precision, spread in 2.87 ms and interpolated in 1.56 ms; here 0.47 and 0.57 ms, bound by the
 // FP64 pipe and, at a quarter of a point per cell, by the latency of the planes that enter and
 // leave the window.
 #include "kernels.cuh"
@@ -22,7 +22,7 @@ void spread_wide_w(const SpreadArgs<T>& a, cudaStream_t stream) {
   const ZChunks ch = make_chunks(i64(a.g.ntiles[0]) * a.g.ntiles[1], a.g.ntiles[2], W);
   const WorkList wl = zwin_work_list(a.g, a.pts, ch);
   dim3 grid{unsigned(wl.grid), unsigned(a.batch), 1u};
-  spread_zwin_kernel<T, W, kWideTx, kWideTy><<<grid, S::NT, 0, stream>>>(a, ch, wl);
+  spread_zwin_wide_kernel<T, W, kWideTx, kWideTy><<<grid, S::NT, 0, stream>>>(a, ch, wl);
   NNB_LAUNCH_CHECK();
 }
 
