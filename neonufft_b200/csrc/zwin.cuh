@@ -410,7 +410,10 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
   // One vector and one plane per thread in single precision keeps the formula: with the
   // polynomials ptxas takes 96 instead of 55 registers and 1e8 points on 480^3 cells 23.5 instead
   // of 16.5 ms (20.2 capped at 64). With two planes they take 1e7 points from 2.32 to 1.86 ms.
-  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || NV > 1 || PZ > 1;
+  // Two vectors take what the single vector of the same tile and width takes: on points clustered
+  // in a few cells the formula's rounding (5e-7 per dimension) does not average out, and the
+  // vectors of transform_type_1_many would differ from single transforms by more than 1e-6.
+  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || PZ > 1 || (NV > 1 && W >= 5 && TY == 8);
   const u32 npts = cta.pend - cta.pbeg;
   const int nbatch = int((npts + S::BATCH - 1) / S::BATCH);
   auto stage = [&](int k) {
