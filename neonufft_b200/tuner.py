@@ -62,7 +62,7 @@ def heuristic_width(tol: float, upsampfac: float, precision: str) -> int:
 def resolved(p: Problem, c: Config):
     """(kernel width, method, x tile, y tile) that a plan with configuration c uses."""
     w = c.n_spread or heuristic_width(p.tol, c.upsampfac, p.precision)
-    method = c.method or (3 if p.dim == 3 and w <= 8 else 1)
+    method = c.method or (3 if p.dim == 3 else 1)
     tile0 = c.tile[0] or (4 if method == 3 else 0)
     tile1 = c.tile[1] or (8 if method == 3 else 0)
     return w, method, tile0, tile1
@@ -71,15 +71,15 @@ def resolved(p: Problem, c: Config):
 def candidates(p: Problem):
     """The heuristic first, then every (upsampfac, width, method, tile) the tuner considers."""
     out = [HEURISTIC]
-    for sigma in (2.0, 1.5):
+    for sigma in (2.0, 1.75, 1.5, 1.25):
         w0 = heuristic_width(p.tol, sigma, p.precision)
         for w in (w0, w0 + 1):
             if w > 16:
                 continue
             if p.dim == 3:
-                methods = [(1, (0, 0, 0))]
+                methods = [(0, (0, 0, 0)), (1, (0, 0, 0))]
                 if w <= 8:
-                    methods = [(3, (8, 8, 1)), (3, (4, 8, 1))] + methods
+                    methods = [(3, (8, 8, 1)), (3, (4, 8, 1)), (1, (0, 0, 0))]
                     if p.precision == "f32" and w >= 5:
                         methods.insert(2, (3, (4, 4, 1)))  # 4-row tiles: single precision
             elif p.dim == 2:
@@ -271,19 +271,35 @@ class Tuner:
             t.model = CostModel.from_state(doc["model"])
         return t
 
+    # candidates that pick() measures past the best-ranked one that meets tol: the default kernels
+    # of close configurations differ by less than the model resolves
+    PICK_MORE = 2
+
     def pick(self, p: Problem, data: ProblemData = None):
-        """(configuration, measured (ms, error), candidates tried): the best-ranked candidate
-        whose measured error meets tol; the heuristic when none does."""
+        """(configuration, measured (ms, error), candidates tried): the fastest of the best-ranked
+        candidate whose measured error meets tol and the PICK_MORE next ones; the heuristic when
+        none meets it."""
         cands = candidates(p)
         if self.model is None:
             return HEURISTIC, None, 0
         pred = self.model.predict(np.stack([features(p, c) for c in cands]))
         data = data or ProblemData(p)
-        for tried, i in enumerate(np.argsort(pred), start=1):
+        best, last = None, len(cands)
+        tried = 0
+        for i in np.argsort(pred):
+            if tried >= last:
+                break
+            tried += 1
             r = measure_or_none(p, cands[int(i)], data)
-            if r is not None and r[1] <= p.tol:
-                return cands[int(i)], r, tried
-        return HEURISTIC, measure(p, HEURISTIC, data), len(cands)
+            if r is None or r[1] > p.tol:
+                continue
+            if best is None:
+                last = min(last, tried + self.PICK_MORE)
+            if best is None or r[0] < best[1][0]:
+                best = (cands[int(i)], r)
+        if best is None:
+            return HEURISTIC, measure(p, HEURISTIC, data), len(cands)
+        return best[0], best[1], tried
 
 
 def rule_plus_one(p: Problem) -> Config:
