@@ -53,16 +53,20 @@ typedef struct NnbOptions {
   int num_threads;          /* ignored on the GPU, as in the reference */
   int sort_input;           /* ignored: points are always bin-sorted */
   int sort_output;          /* ignored: points are always bin-sorted */
-  int kernel_approximation; /* ignored: the ES kernel is always evaluated directly */
+  int kernel_approximation; /* ignored: kernel values always have the precision of the plan */
   int order;                /* NeonufftModeOrder */
   int kernel_type;          /* NeonufftKernelType */
   int tile[3];              /* subproblem tile (bin) shape in fine-grid cells; 0 = automatic.
                                Method 3 takes {2|4|8, 8|16, 1} (16 rows: single precision) and
                                {4, 4, 1} (single precision); the default is {4, 8, 1}.
                                Method 5 uses {4, 4, 1} */
-  int spread_method;        /* 0 = automatic (3 for 3D plans with kernel width <= 8, else 1);
-                               1 = warp-private shared-memory slabs; 2 = thread per point;
-                               3 = sliding z-window held in registers (3D, width <= 8);
+  int spread_method;        /* 0 = automatic (3 for 3D plans, else 1; 1 for 3D plans of kernel
+                               width above 8 that name a tile or have 2^24 planes or more);
+                               1 = 1D and 2D: points along strips, a window of rows held in
+                               registers; 3D, or with a tile: warp-private shared-memory slabs;
+                               2 = thread per point;
+                               3 = sliding z-window held in registers (3D; on request only for
+                               widths <= 8);
                                4 = method 3 with the row updates on the tensor cores (TF32 with
                                split operands; 3D, single precision, width 5 to 8);
                                5 = spreading on the tcgen05 tensor cores with the region's

@@ -3,7 +3,7 @@
 // Replaces the reference's atomic spreading (src/neonufft/gpu/kernels/spreading_kernel.cu:477-715),
 // which issues 2 w^d global float atomics per point.
 //
-// Method 1 (default), warp-private slabs:
+// Method 1 in 3D, or with an explicit tile (1D and 2D otherwise: strip.cu), warp-private slabs:
 //  * A CTA of up to 4 warps covers as many consecutive tiles (bins) along the last dimension;
 //    each warp owns one tile and a private shared-memory slab holding that tile plus its
 //    (w-1)-cell halo (padded strides chosen to spread lanes over the banks, tile_layout.cuh).
