@@ -317,26 +317,21 @@ constexpr i64 kScanSmall = kScanSmallThreads * kScanItems;
 __global__ void __launch_bounds__(kScanSmallThreads)
     scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out) {
   __shared__ u64 total;
-  u64 carry = 0;
-  for (i64 off = 0; off < n; off += kScanSmallThreads * kScanItems) {
-    const i64 base = off + threadIdx.x * kScanItems;
-    u32 v[kScanItems];
-    u64 s = 0;
+  const i64 base = threadIdx.x * kScanItems;
+  u32 v[kScanItems];
+  u64 s = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      v[k] = scan_input(in, base, k, n, n8);
-      s += v[k];
-    }
-    u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total) + carry;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (base + k < n) out[base + k] = u32(run);
-      run += v[k];
-    }
-    carry += total;
-    __syncthreads();
+  for (int k = 0; k < kScanItems; ++k) {
+    v[k] = scan_input(in, base, k, n, n8);
+    s += v[k];
   }
-  if (threadIdx.x == 0) out[n] = u32(carry);
+  u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total);
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    if (base + k < n) out[base + k] = u32(run);
+    run += v[k];
+  }
+  if (threadIdx.x == 0) out[n] = u32(total);
 }
 
 // Whether a record array starts on a 32-byte boundary (a user allocator may return less), so

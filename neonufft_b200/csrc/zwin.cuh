@@ -321,7 +321,8 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
                                                  const WorkList& wl, u32 item, int batch,
                                                  ZSpreadShared<T, W, TX, TY, NV, PZ>& sh) {
   static_assert(NV == 1 || NV == 2, "one or two strength vectors per pass");
-  static_assert(NV == 1 || PZ == 1, "two vectors use one plane per thread");
+  static_assert(NV == 1 || (PZ == 1 && !ZShape<T, W, TX, TY, PZ>::WIDE),
+                "two vectors use one plane per thread, widths up to 8");
   using S = ZShape<T, W, TX, TY, PZ>;
   using Ops = Packed<T>;
   using P = typename Ops::P;
@@ -522,15 +523,9 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
           const u32 run = m & __ballot_sync(0xffffffffu, pl[h] == tp);
           m &= ~run;
           if (tp != cur) {  // advance the window: planes [cur, tp) are complete
-            if constexpr (S::WIDE) {
-              if (dz < tp - cur) flush(Z0{}, cur + dz);
-            } else {  // (by dz < tp - cur as above: 4 % slower)
-              const int n = min(tp - cur, S::RZ);
-              for (int i = 0; i < n; ++i) {
-                const int r = (cur + i) & (S::RZ - 1);
-                if (th.rb == r) flush(Z0{}, cur + i);
-                if (PZ > 1 && th.rb + S::ZL == r) flush(Z1{}, cur + i);
-              }
+            const int n = min(tp - cur, S::RZ);  // (by dz < tp - cur as for wide kernels: 4 % slower)
+            for (int i = 0; i < n; ++i) {
+              if (th.rb == ((cur + i) & (S::RZ - 1))) flush(Z0{}, cur + i);
             }
             cur = tp;
             dz = S::offset(th.rb, cur);
