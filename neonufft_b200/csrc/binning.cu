@@ -290,8 +290,18 @@ __global__ void __launch_bounds__(kScanThreads) scan_top_kernel(u32* block_sums,
   if (threadIdx.x == 0) block_sums[nb] = u32(carry);
 }
 
+// Adds the points of crowded bins to *points (strip.cu).
+__device__ __forceinline__ void count_crowded(const u32 (&v)[kScanItems], u32* points) {
+  u32 c = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) c += v[k] >= kCrowdedBin ? v[k] : 0u;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (c > 0 && (threadIdx.x & 31) == 0) atomicAdd(points, c);
+}
+
 __global__ void __launch_bounds__(kScanThreads)
-    scan_apply_kernel(const u32* in, i64 n, i64 n8, const u32* block_offsets, i64 nb, u32* out) {
+    scan_apply_kernel(const u32* in, i64 n, i64 n8, const u32* block_offsets, i64 nb, u32* out,
+                      u32* crowded) {
   const i64 base = i64(blockIdx.x) * kScanChunk + threadIdx.x * kScanItems;
   u32 v[kScanItems];
   u64 s = 0;
@@ -300,6 +310,7 @@ __global__ void __launch_bounds__(kScanThreads)
     v[k] = scan_input(in, base, k, n, n8);
     s += v[k];
   }
+  if (crowded) count_crowded(v, crowded);
   __shared__ u64 total;
   u64 run = block_exclusive_scan<kScanThreads>(s, &total) + block_offsets[blockIdx.x];
 #pragma unroll
@@ -315,7 +326,7 @@ __global__ void __launch_bounds__(kScanThreads)
 constexpr int kScanSmallThreads = 1024;
 constexpr i64 kScanSmall = kScanSmallThreads * kScanItems;
 __global__ void __launch_bounds__(kScanSmallThreads)
-    scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out) {
+    scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out, u32* crowded) {
   __shared__ u64 total;
   const i64 base = threadIdx.x * kScanItems;
   u32 v[kScanItems];
@@ -325,6 +336,7 @@ __global__ void __launch_bounds__(kScanSmallThreads)
     v[k] = scan_input(in, base, k, n, n8);
     s += v[k];
   }
+  if (crowded) count_crowded(v, crowded);
   u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total);
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
@@ -364,12 +376,12 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
 i64 scan_tmp_words(i64 n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
 void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
-                           bool runs) {
+                           bool runs, u32* crowded) {
   const i64 n8 = runs ? count_run(n) : 0;
   const i64 nb = (n + kScanChunk - 1) / kScanChunk;
   if (nb <= 0) return;
   if (n <= kScanSmall) {
-    scan_small_kernel<<<1, kScanSmallThreads, 0, stream>>>(counts, n, n8, out);
+    scan_small_kernel<<<1, kScanSmallThreads, 0, stream>>>(counts, n, n8, out, crowded);
     NNB_LAUNCH_CHECK();
     return;
   }
@@ -377,7 +389,8 @@ void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStr
   NNB_LAUNCH_CHECK();
   scan_top_kernel<<<1, kScanThreads, 0, stream>>>(tmp, nb);
   NNB_LAUNCH_CHECK();
-  scan_apply_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, n8, tmp, nb, out);
+  scan_apply_kernel<<<unsigned(nb), kScanThreads, 0, stream>>>(counts, n, n8, tmp, nb, out,
+                                                               crowded);
   NNB_LAUNCH_CHECK();
 }
 

@@ -18,10 +18,12 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
                       int* err_flag, cudaStream_t stream);
 // Exclusive scan of n counts into out[0..n] (out[n] = total). tmp needs scan_tmp_words(n).
 i64 scan_tmp_words(i64 n);
-// runs: the counts lie in eight runs of count_run(n), as launch_bin_count leaves them.
+// runs: the counts lie in eight runs of count_run(n), as launch_bin_count leaves them. crowded: if
+// not null, *crowded gets the points in bins of kCrowdedBin points or more added.
+constexpr u32 kCrowdedBin = 8;
 __host__ __device__ __forceinline__ i64 count_run(i64 n) { return (n + 7) / 8; }
 void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
-                           bool runs = false);
+                           bool runs = false, u32* crowded = nullptr);
 // Pass 2: one 32-byte record per point (permutation, packed cell, fractions) in tile order.
 template <typename T>
 void launch_perm_checksum(const PointRec<T>* rec, i64 M, unsigned long long* sums,
@@ -98,6 +100,12 @@ void launch_spread_zwin_wide(const SpreadArgs<T>& a, cudaStream_t stream);
 // 1D and 2D spreading of strip-ordered points (strip.cu).
 template <typename T>
 void launch_spread_strip(const SpreadArgs<T>& a, cudaStream_t stream);
+// Whether M strip-ordered points are so sparse on average that spreading adds their footprints
+// directly, and the flags of the places where they are not (SortedPoints::crowded).
+bool strip_sparse(const BinGeom& g, i64 M);
+template <typename T>
+void launch_strip_crowded(const BinGeom& g, const PointRec<T>* rec, i64 M, unsigned char* crowded,
+                          cudaStream_t stream);
 // Method 5: 3D single-precision spreading on the tcgen05 tensor cores (spread_tc.cu).
 void launch_spread_tc(const SpreadArgs<float>& a, cudaStream_t stream);
 // Status word of the tensor-core spreading: nonzero once one of its bounded waits gave up

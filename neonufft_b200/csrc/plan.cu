@@ -565,7 +565,7 @@ public:
     const BinGeom g = make_geom(dim_, kp_.w, nfft_, tile, D_, scale, bin_order(method_, strips));
     {
       ScopedStage st(timer_, stream_, NNB_STAGE_BIN);
-      out_points_.build(g, s, K, stream_);
+      out_points_.build(g, s, K, stream_, false);
     }
     ScopedStage st(timer_, stream_, NNB_STAGE_PHASE);
     postphase_.reserve(size_t(K));

@@ -329,10 +329,11 @@ template class FftGrid<double>;
 template <typename T>
 PointSet<T>::PointSet(std::shared_ptr<DeviceAllocator> alloc)
     : rec_(alloc), counts_(alloc), bin_start_(alloc), ranks_(alloc), scan_tmp_(alloc),
-      work_start_(alloc), work_owner_(alloc), checksum_(alloc) {}
+      work_start_(alloc), work_owner_(alloc), crowded_(alloc), checksum_(alloc) {}
 
 template <typename T>
-void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream) {
+void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream,
+                        bool spread) {
   if (M < 0) throw_input("negative number of points");
   if (M > i64(0xffffffffll)) throw_input("more than 2^32 - 1 points per plan");
   for (int d = 0; d < g.dim && M > 0; ++d) {
@@ -340,9 +341,11 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   }
   g_ = g;
   M_ = M;
+  crowded_points_ = 0;
   const i64 nt = g.total_tiles;
   const i64 nc = 8 * count_run(nt);
-  counts_.reserve(size_t(nc + 1));  // the error flag behind the counts: one memset for both
+  // behind the counts the error flag and the points of crowded bins: one memset for all
+  counts_.reserve(size_t(nc + 2));
   bin_start_.reserve(size_t(nt + 1));
   scan_tmp_.reserve(size_t(scan_tmp_words(nt)));
   rec_.reserve(size_t(M));
@@ -353,15 +356,17 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
     work_start_.reserve(size_t(nt + 1));
     work_owner_.reserve(size_t(nt + M / kWorkItemPoints + 2));
   }
-  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nc + 1), stream));
+  NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nc + 2), stream));
   int* err = reinterpret_cast<int*>(counts_.data() + nc);
   launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err, stream);
-  launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream, true);
+  const bool sparse = spread && strip_sparse(g, M);
+  launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream, true,
+                        sparse ? counts_.data() + nc + 1 : nullptr);
   launch_bin_scatter<T>(g, x, M, ranks_.data(), bin_start_.data(), rec_.data(), stream);
   // every z-window transform of these points walks the same list of work items
   if (g.zmajor && M > 0) zwin_build_work_list<T>(g, view(), stream);
-  int host_err = 0;
-  NNB_CUDA(cudaMemcpyAsync(&host_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  u32 host[2] = {0, 0};
+  NNB_CUDA(cudaMemcpyAsync(host, err, sizeof(host), cudaMemcpyDeviceToHost, stream));
 #ifdef NNB_CHECKED
   // The records' permutation must be 0 .. M - 1, each once: compare its sum and sum of squares
   // (wrapping 64-bit, as the device adds them) with the closed forms.
@@ -371,7 +376,7 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   NNB_CUDA(cudaMemcpyAsync(sums, checksum_.data(), sizeof(sums), cudaMemcpyDeviceToHost, stream));
 #endif
   NNB_CUDA(cudaStreamSynchronize(stream));
-  if (host_err) {
+  if (host[0]) {
     M_ = 0;
     throw_input("non-finite point coordinate");
   }
@@ -385,6 +390,13 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
     throw_internal("checked build: the bin-sorted records are not a permutation of the points");
   }
 #endif
+  // up to as many points as the shared-memory kernels' work items hold need no windows
+  if (host[1] > kWorkItemPoints) {
+    crowded_.reserve(size_t((M + kStripUnit - 1) / kStripUnit));
+    launch_strip_crowded<T>(g, rec_.data(), M, crowded_.data(), stream);
+    NNB_CUDA(cudaStreamSynchronize(stream));
+    crowded_points_ = host[1];
+  }
 }
 
 template <typename T>
@@ -399,6 +411,8 @@ SortedPoints<T> PointSet<T>::view() const {
   v.work.max_units = g_.total_tiles;
   v.work.max_items = g_.total_tiles + M_ / kWorkItemPoints + 2;
   v.bin_start = bin_start_.data();
+  v.crowded = crowded_.data();
+  v.crowded_points = crowded_points_;
   return v;
 }
 

@@ -167,8 +167,8 @@ public:
   explicit PointSet(std::shared_ptr<DeviceAllocator> alloc);
   // Bins M points; enqueues work on `stream`, then synchronises it and throws InputError for
   // non-finite coordinates (and, in the checked build, InternalError when the records' point
-  // indices are not a permutation of 0 .. M - 1).
-  void build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream);
+  // indices are not a permutation of 0 .. M - 1). spread: the points are spread from, too.
+  void build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream, bool spread = true);
   SortedPoints<T> view() const;
   i64 size() const { return M_; }
   const BinGeom& geom() const { return g_; }
@@ -178,6 +178,8 @@ private:
   i64 M_ = 0;
   DevArray<PointRec<T>> rec_;
   DevArray<u32> counts_, bin_start_, ranks_, scan_tmp_, work_start_, work_owner_;
+  DevArray<unsigned char> crowded_;  // SortedPoints::crowded
+  i64 crowded_points_ = 0;
   DevArray<unsigned long long> checksum_;  // checked build: permutation checksum of the records
 };
 

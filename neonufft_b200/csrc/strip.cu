@@ -41,6 +41,7 @@ namespace {
 
 constexpr int kStripWarps = 4;          // warps per CTA (spreading)
 constexpr int kStripInterpThreads = 128;
+static_assert(32 * kStripWarps == kStripUnit, "direct spreading: one CTA per unit of points");
 
 template <typename T, int DIM, int W>
 struct StripShape {
@@ -86,26 +87,30 @@ __device__ __forceinline__ void strip_cell(const PointRec<T>& r, int& x0, int& y
   y0 = DIM == 2 ? strip_row(r) : 0;
 }
 
-template <typename T, int DIM, int W>
-__global__ void __launch_bounds__(32 * kStripWarps)
-    spread_strip_kernel(const __grid_constant__ SpreadArgs<T> a, u32 chunk) {
+// Spreads the runs of CTA `block`. UNITS: of the points in the units flagged as crowded only.
+template <typename T, int DIM, int W, bool UNITS = false>
+__device__ __forceinline__ void spread_strip_runs(const SpreadArgs<T>& a, u32 chunk, u32 block,
+                                                  StripSlot<T, DIM, W> (*slots)[32]) {
   using S = StripShape<T, DIM, W>;
   using Ops = Packed<T>;
   using P = typename Ops::P;
   using C = cplx_t<T>;
   constexpr int RY = S::RY;
-  __shared__ StripSlot<T, DIM, W> slots[kStripWarps][32];
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int grp = lane / RY;
   const int rb = lane % RY;
   const i64 M = a.pts.M;
-  const i64 first = (i64(blockIdx.x) * kStripWarps + warp) * S::NG * chunk;  // of the warp
+  const i64 first = (i64(block) * kStripWarps + warp) * S::NG * chunk;  // of the warp
   if (first >= M) return;
   const i64 beg = first + i64(grp) * chunk;
   // lanes left over by the runs have no points
-  const int count = grp < S::NG ? int(max(i64(0), min(i64(chunk), M - beg))) : 0;
+  int count = grp < S::NG ? int(max(i64(0), min(i64(chunk), M - beg))) : 0;
+  if constexpr (UNITS) {  // chunk divides the unit
+    if (count > 0 && a.pts.crowded[beg / kStripUnit] == 0) count = 0;
+    if (!__any_sync(0xffffffffu, count > 0)) return;
+  }
   // run 0 of a warp is its longest
   const int iters = (int(min(i64(chunk), M - first)) + RY - 1) / RY;
 
@@ -254,11 +259,18 @@ __global__ void __launch_bounds__(32 * kStripWarps)
   flush(i64(cur) + dz);
 }
 
+template <typename T, int DIM, int W>
+__global__ void __launch_bounds__(32 * kStripWarps)
+    spread_strip_kernel(const __grid_constant__ SpreadArgs<T> a, u32 chunk) {
+  __shared__ StripSlot<T, DIM, W> slots[kStripWarps][32];
+  spread_strip_runs<T, DIM, W>(a, chunk, blockIdx.x, slots);
+}
+
 // 2D spreading of points so sparse that a window's rows would be flushed after a point or two: the
 // warp's lanes add a point's footprint to the grid directly, neighbouring lanes neighbouring
 // cells, so that one atomic instruction covers whole sectors of several rows. An element is an
 // aligned pair of cells (16 bytes) in single precision, a real or imaginary part in double (there
-// are no vector atomics for doubles).
+// are no vector atomics for doubles). A CTA takes one unit of points.
 template <typename T, int W>
 struct SparseShape {
   static constexpr bool SINGLE = sizeof(T) == 4;
@@ -275,15 +287,14 @@ struct SparseSlot {
 };
 
 template <typename T, int W>
-__global__ void __launch_bounds__(32 * kStripWarps)
-    spread_sparse_kernel(const __grid_constant__ SpreadArgs<T> a, bool aligned) {
+__device__ __forceinline__ void spread_sparse_unit(const SpreadArgs<T>& a, bool aligned, u32 unit,
+                                                   SparseSlot<T, W> (*slots)[32]) {
   using S = SparseShape<T, W>;
   using C = cplx_t<T>;
-  __shared__ SparseSlot<T, W> slots[kStripWarps][32];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const i64 M = a.pts.M;
-  const i64 first = (i64(blockIdx.x) * kStripWarps + warp) * 32;
+  const i64 first = i64(unit) * kStripUnit + warp * 32;
   if (first >= M) return;
   const int count = int(min(i64(32), M - first));
   const C* __restrict__ in = a.in + i64(blockIdx.y) * a.in_bdist;
@@ -361,6 +372,33 @@ __global__ void __launch_bounds__(32 * kStripWarps)
   }
 }
 
+template <typename T, int W>
+__global__ void __launch_bounds__(32 * kStripWarps)
+    spread_sparse_kernel(const __grid_constant__ SpreadArgs<T> a, bool aligned) {
+  __shared__ SparseSlot<T, W> slots[kStripWarps][32];
+  spread_sparse_unit<T, W>(a, aligned, blockIdx.x, slots);
+}
+
+// Sparse points with crowded units: the first `nwindow` CTAs walk the crowded ones through windows
+// in runs of `chunk` points, the others add the points of the rest directly. (One launch, so that
+// the latency of a few runs hides behind the direct additions: 1e6 radial points on 3000^2 cells,
+// w = 7, 97 us; 127 in two launches, 106 with all points added directly.)
+template <typename T, int W>
+__global__ void __launch_bounds__(32 * kStripWarps)
+    spread_mixed_kernel(const __grid_constant__ SpreadArgs<T> a, bool aligned, u32 chunk,
+                        u32 nwindow) {
+  __shared__ union Slots {
+    __device__ Slots() {}
+    StripSlot<T, 2, W> window[kStripWarps][32];
+    SparseSlot<T, W> direct[kStripWarps][32];
+  } sh;
+  if (blockIdx.x < nwindow) {
+    spread_strip_runs<T, 2, W, true>(a, chunk, blockIdx.x, sh.window);
+  } else if (a.pts.crowded[blockIdx.x - nwindow] == 0) {
+    spread_sparse_unit<T, W>(a, aligned, blockIdx.x - nwindow, sh.direct);
+  }
+}
+
 template <typename T, int DIM, int W>
 __global__ void __launch_bounds__(kStripInterpThreads)
     interp_strip_kernel(const __grid_constant__ InterpArgs<T> a) {
@@ -434,25 +472,56 @@ u32 strip_chunk(i64 M, int runs_per_warp, int ry) {
   return u32(c < lo ? lo : (c > hi ? hi : c));
 }
 
-// Whether the points of a 2D grid are too sparse for windows: w cells per point or more, at least
-// 6. Uniform points on 4096^2 cells (2048^2 in double precision), windows / direct, in us, at 20,
-// 10 and 5 cells per point: w = 4 133 / 75, 173 / 119, 209 / 223; w = 8 193 / 126, 232 / 212,
-// 344 / 405; double w = 10 138 / 79, 174 / 147, 249 / 290; w = 13 177 / 123, 218 / 239, 303 / 495.
-// The type-3 spread of 5e6 points on 12740^2 cells, w = 6: 2176 / 827 (shared-memory slabs 1335).
-bool sparse_points(const BinGeom& g, i64 M) {
-  return double(M) * std::max(6, g.w) < double(g.nf[0]) * double(g.nf[1]);
+// Whether a unit of points is crowded: four or more of its points to every bin that it touches.
+// (Uniform points at the limit to sparse sets come 1.2 to 1.8 to an occupied bin.)
+template <typename T>
+__global__ void __launch_bounds__(kStripUnit)
+    strip_crowded_kernel(const PointRec<T>* __restrict__ rec, i64 M, int tx,
+                         unsigned char* crowded) {
+  const i64 i = i64(blockIdx.x) * kStripUnit + threadIdx.x;
+  bool first = false;
+  if (i < M) {
+    int x0, y0;
+    strip_cell<2>(rec[i], x0, y0);
+    first = threadIdx.x == 0;
+    if (!first) {
+      int px, py;
+      strip_cell<2>(rec[i - 1], px, py);
+      first = py != y0 || px / tx != x0 / tx;
+    }
+  }
+  const int bins = __syncthreads_count(first);
+  if (threadIdx.x == 0) {
+    const int n = int(min(i64(kStripUnit), M - i64(blockIdx.x) * kStripUnit));
+    crowded[blockIdx.x] = 4 * bins <= n ? 1 : 0;
+  }
 }
 
 template <typename T, int DIM, int W>
 void launch_spread_strip_w(const SpreadArgs<T>& a, cudaStream_t stream) {
   using S = StripShape<T, DIM, W>;
   if constexpr (DIM == 2) {
-    if (sparse_points(a.g, a.pts.M)) {
-      const i64 ctas = (a.pts.M + 32 * kStripWarps - 1) / (32 * kStripWarps);
+    const i64 ctas = (a.pts.M + kStripUnit - 1) / kStripUnit;  // units
+    if (strip_sparse(a.g, a.pts.M)) {
       const bool aligned = a.g.nf[0] % 2 == 0 && a.grid_bdist % 2 == 0 &&
                            reinterpret_cast<uintptr_t>(a.grid) % 16 == 0;
       dim3 grid{unsigned(ctas), unsigned(a.batch), 1u};
-      spread_sparse_kernel<T, W><<<grid, 32 * kStripWarps, 0, stream>>>(a, aligned);
+      // The crowded units go to windows: added directly, the points of a cluster queue up for a
+      // few sectors, and a cell's sum is rounded once per point (1.2e6 points of one sign, sigma
+      // 0.01 rad, 3000^2 cells, w = 7: 1669 us and a relative error of 2e-4 against 78 us and
+      // 9e-7).
+      if (a.pts.crowded_points == 0) {
+        spread_sparse_kernel<T, W><<<grid, 32 * kStripWarps, 0, stream>>>(a, aligned);
+      } else {
+        // runs of a unit; of a half or a quarter while there are few
+        u32 chunk = kStripUnit;
+        while (chunk > 32 && a.pts.crowded_points / chunk < 148 * 24) chunk /= 2;
+        const i64 per_cta = i64(chunk) * S::NG * kStripWarps;
+        const unsigned nwindow = unsigned((a.pts.M + per_cta - 1) / per_cta);
+        grid.x += nwindow;
+        spread_mixed_kernel<T, W><<<grid, 32 * kStripWarps, 0, stream>>>(a, aligned, chunk,
+                                                                         nwindow);
+      }
       NNB_LAUNCH_CHECK();
       return;
     }
@@ -492,6 +561,23 @@ void check_strip_geom(const BinGeom& g) {
 
 }  // namespace
 
+// w cells per point or more, at least 6. Uniform points on 4096^2 cells (2048^2 in double
+// precision), windows / direct, in us, at 20, 10 and 5 cells per point: w = 4 133 / 75, 173 / 119,
+// 209 / 223; w = 8 193 / 126, 232 / 212, 344 / 405; double w = 10 138 / 79, 174 / 147, 249 / 290;
+// w = 13 177 / 123, 218 / 239, 303 / 495. The type-3 spread of 5e6 points on 12740^2 cells, w = 6:
+// 2176 / 827 (shared-memory slabs 1335).
+bool strip_sparse(const BinGeom& g, i64 M) {
+  return g.dim == 2 && g.strip && double(M) * std::max(6, g.w) < double(g.nf[0]) * double(g.nf[1]);
+}
+
+template <typename T>
+void launch_strip_crowded(const BinGeom& g, const PointRec<T>* rec, i64 M, unsigned char* crowded,
+                          cudaStream_t stream) {
+  const i64 units = (M + kStripUnit - 1) / kStripUnit;
+  strip_crowded_kernel<T><<<unsigned(units), kStripUnit, 0, stream>>>(rec, M, g.tile[0], crowded);
+  NNB_LAUNCH_CHECK();
+}
+
 template <typename T>
 void launch_spread_strip(const SpreadArgs<T>& a, cudaStream_t stream) {
   check_strip_geom(a.g);
@@ -527,6 +613,10 @@ void launch_interp_strip(const InterpArgs<T>& a, cudaStream_t stream) {
 
 template void launch_spread_strip<float>(const SpreadArgs<float>&, cudaStream_t);
 template void launch_spread_strip<double>(const SpreadArgs<double>&, cudaStream_t);
+template void launch_strip_crowded<float>(const BinGeom&, const PointRec<float>*, i64,
+                                          unsigned char*, cudaStream_t);
+template void launch_strip_crowded<double>(const BinGeom&, const PointRec<double>*, i64,
+                                           unsigned char*, cudaStream_t);
 template void launch_interp_strip<float>(const InterpArgs<float>&, cudaStream_t);
 template void launch_interp_strip<double>(const InterpArgs<double>&, cudaStream_t);
 

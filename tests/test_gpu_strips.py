@@ -71,6 +71,30 @@ def test_clusters(dtype, type_, modes, cuda, engine, oracle):
     _check(engine, cuda, oracle, dtype, 6, type_, pts, modes)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", [2, 5, 7, 8, 11])
+@pytest.mark.parametrize("share", [1.0, 0.6, 0.05])
+def test_clusters_on_sparse_grids(dtype, w, share, cuda, engine, oracle):
+    """Points that are sparse on average (17 cells a point) of which a share lies in a few cells:
+    the crowded places go through windows, the rest is added directly, and all through windows
+    where nearly all is crowded. Against the thread-per-point method in double precision."""
+    rng = np.random.default_rng(w)
+    M, modes = 400_003, [1300, 1301]
+    n = int(share * M)
+    pts = [np.concatenate([0.7 + 0.005 * rng.standard_normal(n),
+                           rng.uniform(-np.pi, np.pi, M - n)]).astype(dtype) for _ in modes]
+    c = rng.uniform(0.5, 1.5, M).astype(dtype).astype(complex)
+    out, info = run_t12(engine, cuda, dtype, 1, pts, c, modes, 1, n_spread=w)
+    assert info["spread_method"] == 1
+    ref, _ = run_t12(engine, cuda, "float64", 1, pts, c, modes, 1, n_spread=w, spread_method=2)
+    # Strengths of one sign, so that sums grow. Single precision: a cell's sum is made of runs of
+    # 64 or 128 values in registers, up to M / 64 = 6250 of them added to the grid: rounding errors
+    # of u = 6e-8 at random in growing sums, u (sqrt(128) + sqrt(6250)) / sqrt(3) = 3.1e-6, and the
+    # kernel values' 3e-7. Added one by one, the 4e5 values leave 6e-6 (a share of 0.05) to 3e-4.
+    # Double precision: 1e-16 in place of u, the values one by one in the reference.
+    assert oracle.rel_l2(out, ref) < (4e-6 if dtype == "float32" else 1e-13)
+
+
 def spectrum_ratio(beta, w, upsampfac):
     x = np.linspace(-w / 2, w / 2, 20001)
     phi = np.exp(beta * (np.sqrt(np.maximum(0, 1 - 4 * x * x / w ** 2)) - 1))
