@@ -290,18 +290,18 @@ __global__ void __launch_bounds__(kScanThreads) scan_top_kernel(u32* block_sums,
   if (threadIdx.x == 0) block_sums[nb] = u32(carry);
 }
 
-// Adds the points of crowded bins to *points (strip.cu).
-__device__ __forceinline__ void count_crowded(const u32 (&v)[kScanItems], u32* points) {
+// Adds the points of crowded bins to *crowded.points (strip.cu).
+__device__ __forceinline__ void count_crowded(const u32 (&v)[kScanItems], CrowdedBins crowded) {
   u32 c = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) c += v[k] >= kCrowdedBin ? v[k] : 0u;
+  for (int k = 0; k < kScanItems; ++k) c += v[k] >= crowded.least ? v[k] : 0u;
   c = __reduce_add_sync(0xffffffffu, c);
-  if (c > 0 && (threadIdx.x & 31) == 0) atomicAdd(points, c);
+  if (c > 0 && (threadIdx.x & 31) == 0) atomicAdd(crowded.points, c);
 }
 
 __global__ void __launch_bounds__(kScanThreads)
     scan_apply_kernel(const u32* in, i64 n, i64 n8, const u32* block_offsets, i64 nb, u32* out,
-                      u32* crowded) {
+                      CrowdedBins crowded) {
   const i64 base = i64(blockIdx.x) * kScanChunk + threadIdx.x * kScanItems;
   u32 v[kScanItems];
   u64 s = 0;
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kScanThreads)
     v[k] = scan_input(in, base, k, n, n8);
     s += v[k];
   }
-  if (crowded) count_crowded(v, crowded);
+  if (crowded.points) count_crowded(v, crowded);
   __shared__ u64 total;
   u64 run = block_exclusive_scan<kScanThreads>(s, &total) + block_offsets[blockIdx.x];
 #pragma unroll
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kScanThreads)
 constexpr int kScanSmallThreads = 1024;
 constexpr i64 kScanSmall = kScanSmallThreads * kScanItems;
 __global__ void __launch_bounds__(kScanSmallThreads)
-    scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out, u32* crowded) {
+    scan_small_kernel(const u32* in, i64 n, i64 n8, u32* out, CrowdedBins crowded) {
   __shared__ u64 total;
   const i64 base = threadIdx.x * kScanItems;
   u32 v[kScanItems];
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kScanSmallThreads)
     v[k] = scan_input(in, base, k, n, n8);
     s += v[k];
   }
-  if (crowded) count_crowded(v, crowded);
+  if (crowded.points) count_crowded(v, crowded);
   u64 run = block_exclusive_scan<kScanSmallThreads>(s, &total);
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
@@ -376,7 +376,7 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
 i64 scan_tmp_words(i64 n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
 
 void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
-                           bool runs, u32* crowded) {
+                           bool runs, CrowdedBins crowded) {
   const i64 n8 = runs ? count_run(n) : 0;
   const i64 nb = (n + kScanChunk - 1) / kScanChunk;
   if (nb <= 0) return;

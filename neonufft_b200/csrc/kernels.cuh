@@ -18,12 +18,15 @@ void launch_bin_count(const BinGeom& g, CoordPtrs<T> x, i64 M, u32* counts, u32*
                       int* err_flag, cudaStream_t stream);
 // Exclusive scan of n counts into out[0..n] (out[n] = total). tmp needs scan_tmp_words(n).
 i64 scan_tmp_words(i64 n);
-// runs: the counts lie in eight runs of count_run(n), as launch_bin_count leaves them. crowded: if
-// not null, *crowded gets the points in bins of kCrowdedBin points or more added.
-constexpr u32 kCrowdedBin = 8;
+// runs: the counts lie in eight runs of count_run(n), as launch_bin_count leaves them. crowded:
+// the points in bins of crowded.least points or more are added to *crowded.points (if not null).
+struct CrowdedBins {
+  u32* points = nullptr;
+  u32 least = 0;
+};
 __host__ __device__ __forceinline__ i64 count_run(i64 n) { return (n + 7) / 8; }
 void launch_exclusive_scan(const u32* counts, u32* out, i64 n, u32* tmp, cudaStream_t stream,
-                           bool runs = false, u32* crowded = nullptr);
+                           bool runs = false, CrowdedBins crowded = {});
 // Pass 2: one 32-byte record per point (permutation, packed cell, fractions) in tile order.
 template <typename T>
 void launch_perm_checksum(const PointRec<T>* rec, i64 M, unsigned long long* sums,

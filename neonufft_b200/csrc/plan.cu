@@ -342,7 +342,7 @@ public:
 private:
   SpreadArgs<T> spread_args(const void* in) const {
     SpreadArgs<T> a{};
-    a.g = geom_;
+    a.g = points_.geom();
     a.pts = points_.view();
     a.in = static_cast<const cplx_t<T>*>(in);
     a.prephase = nullptr;
@@ -359,7 +359,7 @@ private:
 
   InterpArgs<T> interp_args(void* out) const {
     InterpArgs<T> a{};
-    a.g = geom_;
+    a.g = points_.geom();
     a.pts = points_.view();
     a.grid = fft_->data();
     a.postphase = nullptr;

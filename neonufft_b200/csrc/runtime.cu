@@ -339,9 +339,30 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   for (int d = 0; d < g.dim && M > 0; ++d) {
     if (!x.p[d]) throw_input("null coordinate pointer");
   }
+  // Points crowded by eight or more to a bin of one row (as many per row of wider bins) are worth
+  // finding, unless they are no more than the shared-memory kernels' work items hold.
+  constexpr u32 kCrowdedBin = 8;
+  crowded_points_ = 0;
+  if (spread && g.strip) {
+    const BinGeom wide = widen_strips(g, M);
+    if (wide.total_tiles < g.total_tiles) {
+      const i64 rows = (g.total_tiles + wide.total_tiles - 1) / wide.total_tiles;
+      if (bin(wide, x, M, stream, u32(kCrowdedBin * rows)) <= kWorkItemPoints) return;
+    }
+  }
+  const u32 crowded = bin(g, x, M, stream, spread && strip_sparse(g, M) ? kCrowdedBin : 0);
+  if (crowded > kWorkItemPoints) {
+    crowded_.reserve(size_t((M + kStripUnit - 1) / kStripUnit));
+    launch_strip_crowded<T>(g, rec_.data(), M, crowded_.data(), stream);
+    NNB_CUDA(cudaStreamSynchronize(stream));
+    crowded_points_ = crowded;
+  }
+}
+
+template <typename T>
+u32 PointSet<T>::bin(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream, u32 crowded) {
   g_ = g;
   M_ = M;
-  crowded_points_ = 0;
   const i64 nt = g.total_tiles;
   const i64 nc = 8 * count_run(nt);
   // behind the counts the error flag and the points of crowded bins: one memset for all
@@ -359,9 +380,8 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nc + 2), stream));
   int* err = reinterpret_cast<int*>(counts_.data() + nc);
   launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err, stream);
-  const bool sparse = spread && strip_sparse(g, M);
   launch_exclusive_scan(counts_.data(), bin_start_.data(), nt, scan_tmp_.data(), stream, true,
-                        sparse ? counts_.data() + nc + 1 : nullptr);
+                        CrowdedBins{crowded ? counts_.data() + nc + 1 : nullptr, crowded});
   launch_bin_scatter<T>(g, x, M, ranks_.data(), bin_start_.data(), rec_.data(), stream);
   // every z-window transform of these points walks the same list of work items
   if (g.zmajor && M > 0) zwin_build_work_list<T>(g, view(), stream);
@@ -390,13 +410,7 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
     throw_internal("checked build: the bin-sorted records are not a permutation of the points");
   }
 #endif
-  // up to as many points as the shared-memory kernels' work items hold need no windows
-  if (host[1] > kWorkItemPoints) {
-    crowded_.reserve(size_t((M + kStripUnit - 1) / kStripUnit));
-    launch_strip_crowded<T>(g, rec_.data(), M, crowded_.data(), stream);
-    NNB_CUDA(cudaStreamSynchronize(stream));
-    crowded_points_ = host[1];
-  }
+  return host[1];
 }
 
 template <typename T>
@@ -542,6 +556,18 @@ bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* 
   if (dim == 1) return nf[0] <= (i64(1) << 26);
   const i64 tx = strip_width(complex_bytes / 2, w);
   return nf[1] <= 0x7fffffff && (nf[0] + tx - 1) / tx <= (i64(1) << 26) / nf[1];
+}
+
+BinGeom widen_strips(const BinGeom& g, i64 M) {
+  BinGeom wide = g;
+  const int grow = g.dim - 1;  // 1D: more cells, 2D: more rows
+  const i64 limit = std::max(i64(1) << 16, 8 * M);
+  while (wide.total_tiles > limit && wide.tile[grow] < 64) {
+    wide.tile[grow] *= 2;
+    wide.ntiles[grow] = int((g.nf[grow] + wide.tile[grow] - 1) / wide.tile[grow]);
+    wide.total_tiles = i64(wide.ntiles[0]) * wide.ntiles[1] * wide.ntiles[2];
+  }
+  return wide;
 }
 
 void strip_tile(int dim, int w, size_t complex_bytes, const i64* nf, i64 interp_only_points,

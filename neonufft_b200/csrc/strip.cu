@@ -224,7 +224,8 @@ __device__ __forceinline__ void spread_strip_runs(const SpreadArgs<T>& a, u32 ch
       const auto& pt = slots[warp][grp * RY + j];
       const int tp = pt.row, ts = pt.strip;
       if (tp != cur || ts != strip) {  // rows [cur, tp), or the whole window, are complete
-        if (dz < (ts == strip ? tp - cur : RY)) flush(i64(cur) + dz);
+        // (1D bins may hold several cells in any order: an earlier cell counts as far ahead)
+        if (unsigned(dz) < (ts == strip ? unsigned(tp - cur) : unsigned(RY))) flush(i64(cur) + dz);
         cur = tp;
         strip = ts;
         dz = S::offset(rb, cur);
@@ -581,8 +582,9 @@ void launch_strip_crowded(const BinGeom& g, const PointRec<T>* rec, i64 M, unsig
 template <typename T>
 void launch_spread_strip(const SpreadArgs<T>& a, cudaStream_t stream) {
   check_strip_geom(a.g);
-  // the window needs the points of a strip row by row (1D: cell by cell)
-  if (a.g.tile[0] != (a.g.dim == 1 ? 1 : strip_width(sizeof(T), a.g.w)) || a.g.tile[1] != 1) {
+  // 2D windows need the points of a strip row by row
+  if (a.g.dim == 2 && (a.g.tile[0] != strip_width(sizeof(T), a.g.w) ||
+                       (a.g.tile[1] != 1 && !strip_sparse(a.g, a.pts.M)))) {
     throw_internal("strip spreading needs bins of one row");
   }
   if (a.batch > 65535) throw_input("batch size above 65535");

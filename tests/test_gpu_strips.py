@@ -95,6 +95,49 @@ def test_clusters_on_sparse_grids(dtype, w, share, cuda, engine, oracle):
     assert oracle.rel_l2(out, ref) < (4e-6 if dtype == "float32" else 1e-13)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", [2, 3, 6, 7, 12, 16])
+@pytest.mark.parametrize("points", ["uniform", "band", "cell"])
+@pytest.mark.parametrize("modes", [[500_003], [1200, 1100]])
+@pytest.mark.parametrize("type_", [1, 2])
+def test_few_points_on_large_grids(dtype, w, points, modes, type_, cuda, engine, oracle):
+    """Few points on a large grid: the strips' bins are widened, so that their number follows that
+    of the points. "band": some of them lie closely, in any order within the wide bins (2 points a
+    cell in 1D); "cell": most of them in one cell, for which the bins are narrowed again."""
+    rng = np.random.default_rng(w)
+    M = 9000
+    near = {"uniform": 0, "band": 4000, "cell": 6000}[points]
+    span = {"uniform": 0, "band": 4e-3 * np.pi if len(modes) == 1 else 0.1, "cell": 1e-6}[points]
+    pts = [np.concatenate([rng.uniform(0.5, 0.5 + span, near), rng.uniform(-4, 4, M - near)])
+           for _ in modes]
+    pts[0][-1], pts[0][-2] = np.pi - 1e-6, -np.pi  # the periodic edge
+    n_in = M if type_ == 1 else int(np.prod(modes))
+    inp = rng.standard_normal(n_in) + 1j * rng.standard_normal(n_in)
+    out, _ = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w)
+    pts = [p.astype(dtype) for p in pts]
+    ref, _ = run_t12(engine, cuda, "float64", 1, pts, inp, modes, type_, n_spread=w,
+                     spread_method=2)
+    # Single precision: sums of up to 6000 values, u sqrt(6000 / 2) = 3.3e-6 at random signs if added
+    # one by one (u = 6e-8), and 16 of them at once at least here: 8e-7; the kernel values' 1e-7 and
+    # the rounding of beta, which both sides deconvolve by their own value
+    assert oracle.rel_l2(out, ref) < (2e-6 if dtype == "float32" else 1e-13)
+
+
+@pytest.mark.parametrize("modes,tile", [([500_003], (512, 0, 0)), ([1200, 1100], (64, 16, 0))])
+def test_bins_follow_the_points(modes, tile, cuda, engine):
+    """A plan of few points holds no more than 64 bytes a point, or the 512 KB of 65536 bins, above
+    what it holds with the tiles of the shared-memory kernels."""
+    M = 9000
+    x = [cuda.rand(M, device="cuda") * 6 - 3 for _ in modes]
+    held = []
+    for t in [(0, 0, 0), tile]:
+        plan = engine.Plan(engine.Options(tol=1e-6, tile=t), -1, M, x, modes)
+        held.append(plan.info()["device_bytes"])
+        plan.close()
+    # one byte of flags per 128 points, the scan's block sums and roundings up besides
+    assert held[0] <= held[1] + max(64 * M, 8 * 65536) + 16384
+
+
 def spectrum_ratio(beta, w, upsampfac):
     x = np.linspace(-w / 2, w / 2, 20001)
     phi = np.exp(beta * (np.sqrt(np.maximum(0, 1 - 4 * x * x / w ** 2)) - 1))
