@@ -307,12 +307,15 @@ struct SortedPoints {
   const u32* bin_start;  // total_tiles + 1 offsets into the records
   i64 M;
   WorkScratch work;
-  // 2D strip-ordered points that are sparse on average: how many lie in crowded bins and, unless
-  // these are too few to matter (0), one flag per kStripUnit records, set where these lie densely.
+  // Strip-ordered points to spread from: how many lie in crowded bins (kCrowdedSparse points or
+  // more in 2D sets that are sparse on average, kCrowdedDense in others), 0 if too few to matter.
+  // Of sparse sets then one flag per kStripUnit records, set where these lie densely.
   i64 crowded_points;
   const unsigned char* crowded;
 };
 constexpr int kStripUnit = 128;
+constexpr u32 kCrowdedSparse = 8;
+constexpr u32 kCrowdedDense = 1u << 16;
 
 // ES kernel (exponential of semicircle): phi(x) = exp(beta * (sqrt(1 - c x^2) - 1)) for
 // |x| < w/2, else 0, c = 4 / w^2 (reference src/neonufft/gpu/kernels/es_kernel_eval.cuh:18-44).

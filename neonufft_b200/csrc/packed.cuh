@@ -29,6 +29,9 @@ struct Packed<float> {
     asm("mov.b64 {_, %0}, %1;" : "=f"(y) : "l"(v));
     return y;
   }
+  static __device__ __forceinline__ P shfl(P v, int lane) {
+    return __shfl_sync(0xffffffffu, v, lane);
+  }
   // a * b + c, elementwise
   static __device__ __forceinline__ P fma(P a, P b, P c) {
     P d;
@@ -50,6 +53,9 @@ struct Packed<double> {
   static __device__ __forceinline__ P splat(double x) { return P{x, x}; }
   static __device__ __forceinline__ double lo(P v) { return v.x; }
   static __device__ __forceinline__ double hi(P v) { return v.y; }
+  static __device__ __forceinline__ P shfl(P v, int lane) {
+    return P{__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane)};
+  }
   static __device__ __forceinline__ P fma(P a, P b, P c) {
     return P{::fma(a.x, b.x, c.x), ::fma(a.y, b.y, c.y)};
   }

@@ -339,24 +339,27 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
   for (int d = 0; d < g.dim && M > 0; ++d) {
     if (!x.p[d]) throw_input("null coordinate pointer");
   }
-  // Points crowded by eight or more to a bin of one row (as many per row of wider bins) are worth
-  // finding, unless they are no more than the shared-memory kernels' work items hold.
-  constexpr u32 kCrowdedBin = 8;
   crowded_points_ = 0;
-  if (spread && g.strip) {
-    const BinGeom wide = widen_strips(g, M);
-    if (wide.total_tiles < g.total_tiles) {
-      const i64 rows = (g.total_tiles + wide.total_tiles - 1) / wide.total_tiles;
-      if (bin(wide, x, M, stream, u32(kCrowdedBin * rows)) <= kWorkItemPoints) return;
-    }
+  if (!spread || !g.strip) {
+    bin(g, x, M, stream, 0);
+    return;
   }
-  const u32 crowded = bin(g, x, M, stream, spread && strip_sparse(g, M) ? kCrowdedBin : 0);
-  if (crowded > kWorkItemPoints) {
+  // crowded points are worth finding if they are more than the shared-memory kernels' work items
+  // hold
+  const BinGeom wide = widen_strips(g, M);
+  if (wide.total_tiles < g.total_tiles) {
+    const i64 rows = (g.total_tiles + wide.total_tiles - 1) / wide.total_tiles;
+    if (bin(wide, x, M, stream, u32(kCrowdedSparse * rows)) <= kWorkItemPoints) return;
+  }
+  const bool sparse = strip_sparse(g, M);
+  const u32 crowded = bin(g, x, M, stream, sparse ? kCrowdedSparse : kCrowdedDense);
+  if (crowded <= kWorkItemPoints) return;
+  if (sparse) {
     crowded_.reserve(size_t((M + kStripUnit - 1) / kStripUnit));
     launch_strip_crowded<T>(g, rec_.data(), M, crowded_.data(), stream);
     NNB_CUDA(cudaStreamSynchronize(stream));
-    crowded_points_ = crowded;
   }
+  crowded_points_ = crowded;
 }
 
 template <typename T>

@@ -138,6 +138,32 @@ def test_bins_follow_the_points(modes, tile, cuda, engine):
     assert held[0] <= held[1] + max(64 * M, 8 * 65536) + 16384
 
 
+@pytest.mark.parametrize("w", [2, 4, 7, 10, 16])
+@pytest.mark.parametrize("modes", [[100], [40, 31]])
+def test_many_points_in_a_few_cells(w, modes, cuda, engine, oracle):
+    """Millions of strengths of one sign in a few cells, single precision: runs are longer and
+    the runs of a warp summed before they go to the grid."""
+    torch = cuda
+    gen = torch.Generator(device="cuda").manual_seed(w)
+    M = 12_000_000
+    pts = [(0.7 + 0.02 * torch.randn(M, generator=gen, device="cuda")) for _ in modes]
+    c = torch.rand(M, generator=gen, device="cuda").to(torch.complex64)
+    out = []
+    for dtype, opt in [(torch.float32, {}), (torch.float64, {"spread_method": 2})]:
+        cd = torch.complex64 if dtype == torch.float32 else torch.complex128
+        plan = engine.Plan(engine.Options(tol=1e-6, n_spread=w, **opt), 1, M,
+                           [x.to(dtype) for x in pts], modes)
+        f = torch.empty(int(np.prod(modes)), dtype=cd, device="cuda")
+        plan.transform_type_1(c.to(cd), f, [1] + modes[:1][:len(modes) - 1])
+        torch.cuda.synchronize()
+        out.append(f.cpu().numpy())
+        plan.close()
+    # A run sums M / (148 24 (32 // w)) values one by one, 211 at w = 2 to 1690 at w = 16, and the
+    # sums of 148 24 = 3552 warps are added to a cell at most: rounding errors of u = 6e-8 at random
+    # in growing sums, u (sqrt(1690) + sqrt(3552)) / sqrt(3) = 3.5e-6; the kernel values' 3e-7
+    assert oracle.rel_l2(out[0], out[1]) < 4e-6
+
+
 def spectrum_ratio(beta, w, upsampfac):
     x = np.linspace(-w / 2, w / 2, 20001)
     phi = np.exp(beta * (np.sqrt(np.maximum(0, 1 - 4 * x * x / w ** 2)) - 1))
