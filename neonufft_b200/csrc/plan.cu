@@ -189,8 +189,8 @@ public:
     }
   }
 
-  // Single precision on the z-window kernels (default or 4-row tiles) spreads the vectors two
-  // at a time: each staged point serves both, into a pair of fine grids; each grid is then
+  // Single precision on the z-window kernels (widths up to 8, default or 4-row tiles) spreads the
+  // vectors two at a time: each staged point serves both, into a pair of fine grids; each grid is then
   // transformed and deconvolved into its output.
   void transform_type_1_many(i64 count, const void* in, i64 in_bdist, void* out, i64 out_bdist,
                              const i64* out_strides) override {
@@ -205,7 +205,7 @@ public:
     if (count > 1 && (in_bdist < M || out_bdist < extent)) {
       throw_input("input / output distances smaller than one vector");
     }
-    const bool pairs = is_single<T>() && method_ == 3 && tile_[0] == 4 &&
+    const bool pairs = is_single<T>() && method_ == 3 && kp_.w <= 8 && tile_[0] == 4 &&
                        (tile_[1] == 8 || tile_[1] == 4) && count > 1 && M > 0;
     if (!pairs) {
       PlanBase::transform_type_1_many(count, in, in_bdist, out, out_bdist, out_strides);

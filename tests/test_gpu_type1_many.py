@@ -63,6 +63,34 @@ def test_many_single_precision_pairs(tile, count, case, cuda, engine, oracle):
         assert oracle.rel_l2(many[v], ref) < bound
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_many_wide_kernels_take_no_further_grids(dtype, cuda, engine, oracle):
+    """Widths above 8 have no two-vector kernel: the transforms run one at a time, on the plan's
+    own grid."""
+    torch = cuda
+    rng = np.random.default_rng(9)
+    rdt, cdt, npc = tdtypes(torch, dtype)
+    modes, M, count = [20, 18, 16], 5000, 3
+    nm = int(np.prod(modes))
+    pts = [rng.uniform(-np.pi, np.pi, M).astype(dtype) for _ in range(3)]
+    vecs = [(rng.standard_normal(M) + 1j * rng.standard_normal(M)).astype(npc)
+            for _ in range(count)]
+    plan = engine.Plan(engine.Options(tol=1e-6, n_spread=10), -1, M,
+                       [torch.from_numpy(p).cuda() for p in pts], modes)
+    held = plan.info()["device_bytes"]
+    out = torch.empty(count * nm, dtype=cdt, device="cuda")
+    plan.transform_type_1_many(torch.from_numpy(np.concatenate(vecs)).cuda(), out, count,
+                               col_strides(modes))
+    torch.cuda.synchronize()
+    assert plan.info()["device_bytes"] == held
+    plan.close()
+    for v in range(count):
+        ref = direct(oracle, 1, -1, pts, vecs[v], modes, dtype)
+        # single precision: rounding, 3e-7 of each kernel value among it; double: width 10
+        assert oracle.rel_l2(out.cpu().numpy()[v * nm:(v + 1) * nm], ref) < \
+            (2e-6 if dtype == "float32" else 1e-8)
+
+
 def test_many_outputs_ordered_on_the_plan_stream(cuda, engine, oracle):
     """The FFTs and deconvolutions of each pair run on the plan's internal stream; work that the
     caller enqueues on the plan's stream right after the call (no host synchronisation) must see
