@@ -43,15 +43,27 @@ __device__ __forceinline__ bool next_fused_item(const Job* jobs, const i64* item
   return true;
 }
 
+// Window planes per thread (ZShape::PZ) of the kernels of one transform.
+template <typename T, int W, int TX, int TY>
+constexpr int zwin_planes = sizeof(T) == 4 && W >= 5 && TX == 4 && TY <= 8 ? 2 : 1;
+
+// Kernel values as the launches of one transform take them, but one plane per thread: 24 type-1
+// transforms of 1e4 to 3e6 points, w = 8, single precision, in 6.36 ms (one plane, 5 CTAs per SM;
+// 6.45 and 6.49 with 6 and 7) against 7.10 to 7.40 (two planes, 8 to 11 CTAs) and 7.00 (the
+// formula, 7 CTAs).
 template <typename T, int W, int TX>
-__global__ void __launch_bounds__(ZShape<T, W, TX>::NT, kSpreadFusedCtas<T>)
+constexpr bool fused_poly = zspread_poly<T, W, 8, 1, zwin_planes<T, W, TX, 8>>;
+
+template <typename T, int W, int TX>
+__global__ void __launch_bounds__(ZShape<T, W, TX>::NT,
+                                  sizeof(T) == 4 && fused_poly<T, W, TX> ? 5 : kSpreadFusedCtas<T>)
     spread_zwin_fused_kernel(const ZSpreadJob<T>* jobs, const i64* item_end, int njobs,
                              i64 total, u32* queue) {
   __shared__ ZSpreadShared<T, W, TX> sh;
   __shared__ ZSpreadJob<T> job;
   u32 local;
   while (next_fused_item(jobs, item_end, njobs, total, queue, job, local)) {
-    spread_zwin_item<T, W, TX>(job.a, job.ch, job.wl, local, 0, sh);
+    spread_zwin_item<T, W, TX, 8, 1, 1, fused_poly<T, W, TX>>(job.a, job.ch, job.wl, local, 0, sh);
     __syncthreads();  // the job record and the slots are rewritten for the next item
   }
 }
@@ -294,10 +306,6 @@ template WorkList zwin_work_list<float>(const BinGeom&, const SortedPoints<float
 template WorkList zwin_work_list<double>(const BinGeom&, const SortedPoints<double>&, ZChunks);
 
 namespace {
-
-// Window planes per thread (ZShape::PZ).
-template <typename T, int W, int TX, int TY>
-constexpr int zwin_planes = sizeof(T) == 4 && W >= 5 && TX == 4 && TY <= 8 ? 2 : 1;
 
 template <typename T, int W, int TX, int TY>
 void launch_spread_zwin_tw(const SpreadArgs<T>& a, cudaStream_t stream) {

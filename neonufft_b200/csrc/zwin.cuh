@@ -311,12 +311,25 @@ struct ZSpreadShared {
   cplx_t<T> v2[2][NV > 1 ? ZShape<T, W, TX, TY, PZ>::BATCH : 1];
 };
 
+// Whether spreading takes kernel values from the polynomials.
+//
+// One vector and one plane per thread in single precision keeps the formula: with the
+// polynomials ptxas takes 96 instead of 55 registers and 1e8 points on 480^3 cells 23.5 instead
+// of 16.5 ms (20.2 capped at 64). With two planes they take 1e7 points from 2.32 to 1.86 ms.
+// Two vectors take what the single vector of the same tile and width takes: on points clustered
+// in a few cells the formula's rounding (5e-7 per dimension) does not average out, and the
+// vectors of transform_type_1_many would differ from single transforms by more than 1e-6.
+template <typename T, int W, int TY, int NV, int PZ>
+constexpr bool zspread_poly =
+    sizeof(T) == 8 || W > 8 || PZ > 1 || (NV > 1 && W >= 5 && TY == 8);
+
 // Spreads work item `item` of batch entries batch .. batch + NV - 1 (one CTA; every thread
 // calls it). With NV = 2 each staged point, its kernel values and the window's bookkeeping
 // serve two strength vectors on the same points (type-3 batches, repeated type-1 transforms):
 // the second vector's row sums sit in their own registers and go to the next grid (at
 // grid_bdist); a missing second entry (an odd batch) is skipped.
-template <typename T, int W, int TX, int TY = 8, int NV = 1, int PZ = 1>
+template <typename T, int W, int TX, int TY = 8, int NV = 1, int PZ = 1,
+          bool POLY = zspread_poly<T, W, TY, NV, PZ>>
 __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks ch,
                                                  const WorkList& wl, u32 item, int batch,
                                                  ZSpreadShared<T, W, TX, TY, NV, PZ>& sh) {
@@ -408,13 +421,6 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
   using Z0 = std::integral_constant<int, 0>;
   using Z1 = std::integral_constant<int, PZ - 1>;
 
-  // One vector and one plane per thread in single precision keeps the formula: with the
-  // polynomials ptxas takes 96 instead of 55 registers and 1e8 points on 480^3 cells 23.5 instead
-  // of 16.5 ms (20.2 capped at 64). With two planes they take 1e7 points from 2.32 to 1.86 ms.
-  // Two vectors take what the single vector of the same tile and width takes: on points clustered
-  // in a few cells the formula's rounding (5e-7 per dimension) does not average out, and the
-  // vectors of transform_type_1_many would differ from single transforms by more than 1e-6.
-  constexpr bool kPoly = sizeof(T) == 8 || S::WIDE || PZ > 1 || (NV > 1 && W >= 5 && TY == 8);
   const u32 npts = cta.pend - cta.pbeg;
   const int nbatch = int((npts + S::BATCH - 1) / S::BATCH);
   auto stage = [&](int k) {
@@ -428,7 +434,7 @@ __device__ __forceinline__ void spread_zwin_item(const SpreadArgs<T>& a, ZChunks
         break;
       }
       // NV = 2: the second vector's strengths at the same points (zeros when it is missing)
-      stage_warp<T, W, TX, true, TY, PZ, kPoly>(slots[k & 1] + th.warp * PW + c0,
+      stage_warp<T, W, TX, true, TY, PZ, POLY>(slots[k & 1] + th.warp * PW + c0,
                                  a.pts.rec + cta.pbeg + off + th.warp * PW + c0,
                                  min(count - c0, 16), in, a.prephase, a.es, a.beta, a.c, th.lane,
                                  a.pts.M, NV > 1 && has2 ? in + a.in_bdist : nullptr,
