@@ -71,7 +71,7 @@ def resolved(p: Problem, c: Config):
 def candidates(p: Problem):
     """The heuristic first, then every (upsampfac, width, method, tile) the tuner considers."""
     out = [HEURISTIC]
-    for sigma in (2.0, 1.75, 1.5, 1.25):
+    for sigma in (2.0, 1.5):
         w0 = heuristic_width(p.tol, sigma, p.precision)
         for w in (w0, w0 + 1):
             if w > 16:
@@ -271,35 +271,19 @@ class Tuner:
             t.model = CostModel.from_state(doc["model"])
         return t
 
-    # candidates that pick() measures past the best-ranked one that meets tol: the default kernels
-    # of close configurations differ by less than the model resolves
-    PICK_MORE = 2
-
     def pick(self, p: Problem, data: ProblemData = None):
-        """(configuration, measured (ms, error), candidates tried): the fastest of the best-ranked
-        candidate whose measured error meets tol and the PICK_MORE next ones; the heuristic when
-        none meets it."""
+        """(configuration, measured (ms, error), candidates tried): the best-ranked candidate
+        whose measured error meets tol; the heuristic when none does."""
         cands = candidates(p)
         if self.model is None:
             return HEURISTIC, None, 0
         pred = self.model.predict(np.stack([features(p, c) for c in cands]))
         data = data or ProblemData(p)
-        best, last = None, len(cands)
-        tried = 0
-        for i in np.argsort(pred):
-            if tried >= last:
-                break
-            tried += 1
+        for tried, i in enumerate(np.argsort(pred), start=1):
             r = measure_or_none(p, cands[int(i)], data)
-            if r is None or r[1] > p.tol:
-                continue
-            if best is None:
-                last = min(last, tried + self.PICK_MORE)
-            if best is None or r[0] < best[1][0]:
-                best = (cands[int(i)], r)
-        if best is None:
-            return HEURISTIC, measure(p, HEURISTIC, data), len(cands)
-        return best[0], best[1], tried
+            if r is not None and r[1] <= p.tol:
+                return cands[int(i)], r, tried
+        return HEURISTIC, measure(p, HEURISTIC, data), len(cands)
 
 
 def rule_plus_one(p: Problem) -> Config:

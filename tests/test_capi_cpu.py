@@ -217,3 +217,26 @@ def test_tuner_rows_round_trip_through_a_file(tmp_path):
     bad.write_text(json.dumps(doc))
     with pytest.raises(ValueError):
         T.Tuner.load(bad)
+
+
+def test_tuner_pick_measures_until_tol_is_met(monkeypatch):
+    """A pick measures the candidates in the model's order and stops at the first that meets tol."""
+    from neonufft_b200 import tuner as T
+    p = T.Problem(dim=3, type=1, M=10 ** 5, N=32, tol=1e-6)
+    cands = T.candidates(p)
+    assert {c.upsampfac for c in cands} == {2.0, 1.5}
+
+    class Model:
+        def predict(self, feats):
+            return np.arange(len(feats))[::-1]  # the last candidate first
+
+    measured = []
+
+    def fake(problem, config, data=None):
+        measured.append(config)
+        return (1.0, 1e-5 if len(measured) < 3 else 1e-7)
+
+    monkeypatch.setattr(T, "measure_or_none", fake)
+    cfg, (ms, err), tried = T.Tuner(Model()).pick(p, data=object())
+    assert measured == [cands[-1], cands[-2], cands[-3]]
+    assert cfg == cands[-3] and err <= p.tol and tried == 3

@@ -59,7 +59,9 @@ def test_mlp_training_converges(cuda, engine):
 # Margins the learned picks must keep on the held-out problems (geometric means of the other
 # configuration's time over the pick's time, where that configuration meets tol).
 MARGIN_VS_HEURISTIC = 1.10
-MARGIN_VS_RULE_PLUS_ONE = 1.05
+# The rule's plan has the default kernels. Over three sets of problems like these the picks are 1.051,
+# 1.085 and 1.062 times as fast; 12 problems timed to about 3 % each leave 1 % of a geometric mean.
+MARGIN_VS_RULE_PLUS_ONE = 1.02
 
 
 def _problems(T, n, seed):
