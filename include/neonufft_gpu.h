@@ -57,6 +57,8 @@ typedef struct NnbOptions {
   int order;                /* NeonufftModeOrder */
   int kernel_type;          /* NeonufftKernelType */
   int tile[3];              /* subproblem tile (bin) shape in fine-grid cells; 0 = automatic.
+                               The tile that a plan reports, named together with the method
+                               that it reports, gives the same plan.
                                Method 3 takes {2|4|8, 8|16, 1} (16 rows: single precision) and
                                {4, 4, 1} (single precision); the default is {4, 8, 1}.
                                Method 5 uses {4, 4, 1} */
@@ -65,8 +67,8 @@ typedef struct NnbOptions {
                                1 = 1D and 2D: points along strips, a window of rows held in
                                registers; 3D, or with a tile: warp-private shared-memory slabs;
                                2 = thread per point;
-                               3 = sliding z-window held in registers (3D; on request only for
-                               widths <= 8);
+                               3 = sliding z-window held in registers (3D; on request for widths
+                               <= 8, or above with the tile {4, 8, 1});
                                4 = method 3 with the row updates on the tensor cores (TF32 with
                                split operands; 3D, single precision, width 5 to 8);
                                5 = spreading on the tcgen05 tensor cores with the region's
@@ -215,7 +217,7 @@ typedef struct NnbPlanInfo {
   double es_beta;      /* ES kernel shape parameter (as used, i.e. rounded to T) */
   int64_t grid[3];     /* FFT grid (fine grid) dims; 1 for unused dims */
   int64_t spread_grid[3]; /* type 3: spread grid dims; type 1/2: equals grid */
-  int tile[3];         /* subproblem tile shape */
+  int tile[3];         /* subproblem tile shape (1D, 2D strips: cells per strip and row) */
   int64_t num_in;      /* points (type 1/2) or sources (type 3) */
   int64_t num_out;     /* type 3 targets */
   int64_t batch_size;

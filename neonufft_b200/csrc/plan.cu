@@ -525,7 +525,7 @@ public:
     } else {
       choose_tile(dim_, kp_.w, sizeof(cplx_t<T>), nf1_, opt_.tile, method_, in_tile_);
     }
-    // the output points' strips depend on their number 
+    // (the output points' strips depend on their number)
     choose_tile(dim_, kp_.w, sizeof(cplx_t<T>), nfft_, opt_.tile, method_, out_tile_);
     NNB_CUDA(cudaStreamSynchronize(stream_));
   }
@@ -560,7 +560,8 @@ public:
     double scale[3];
     for (int d = 0; d < 3; ++d) scale[d] = d < dim_ ? gamma_[d] * h_[d] : 1.0;
     int tile[3] = {out_tile_[0], out_tile_[1], out_tile_[2]};
-    const bool strips = method_ == 1 && dim_ < 3 && !(opt_.tile[0] > 0);
+    const bool strips = method_ == 1 && dim_ < 3 &&
+                        strip_tile_or_none(dim_, kp_.w, sizeof(cplx_t<T>), opt_.tile);
     if (strips) strip_tile(dim_, kp_.w, sizeof(cplx_t<T>), nfft_, K > 0 ? K : 1, tile);
     const BinGeom g = make_geom(dim_, kp_.w, nfft_, tile, D_, scale, bin_order(method_, strips));
     {

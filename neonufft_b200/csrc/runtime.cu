@@ -438,7 +438,9 @@ template class PointSet<double>;
 
 // ---- tiles ----------------------------------------------------------------------------------------
 int choose_method(int dim, int w, int requested, bool single, const int* tile, const i64* nf) {
-  if (requested == 3 && (dim != 3 || w > 8)) {
+  // the tile of the wide kernels, as plans report it
+  const bool wide_tile = tile && tile[0] == 4 && tile[1] == 8;
+  if (requested == 3 && (dim != 3 || (w > 8 && !wide_tile))) {
     throw_input("spread method 3 needs a 3D plan with kernel width <= 8");
   }
   if (requested == 4 && (dim != 3 || w < 5 || w > 8 || !single)) {
@@ -552,9 +554,15 @@ void choose_tile(int dim, int w, size_t complex_bytes, const i64* nf, const int*
   }
 }
 
+bool strip_tile_or_none(int dim, int w, size_t complex_bytes, const int* requested) {
+  if (!requested || requested[0] <= 0) return true;
+  if (dim == 1) return requested[0] == 1;
+  return dim == 2 && requested[0] == strip_width(complex_bytes / 2, w) && requested[1] == 1;
+}
+
 bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
                 int method) {
-  if (method != 1 || dim > 2 || (requested && requested[0] > 0)) return false;
+  if (method != 1 || dim > 2 || !strip_tile_or_none(dim, w, complex_bytes, requested)) return false;
   // one bin per strip and row: beyond 2^26 bins (256 MB of counts) the slab tiles stay cheaper
   if (dim == 1) return nf[0] <= (i64(1) << 26);
   const i64 tx = strip_width(complex_bytes / 2, w);

@@ -190,8 +190,9 @@ private:
 
 // Spreading / interpolation method for a plan: the requested one (validated), or the default:
 // 3 (z-window, zwin.cu) for 3D plans, else 1 (strips, or shared-memory slabs). A 3D plan with
-// n_spread > 8 keeps the slabs when it names a tile or has 2^24 planes or more (nf, which may be
-// null as long as it is not known). Method 4 is the z-window with tensor-core spreading (single
+// n_spread > 8 keeps the slabs when it names a tile without a method, or has 2^24 planes or more
+// (nf, which may be null as long as it is not known); it may name method 3 with the tile that the
+// automatic choice reports, {4, 8, 1}. Method 4 is the z-window with tensor-core spreading (single
 // precision, 5 <= n_spread <= 8).
 int choose_method(int dim, int w, int requested, bool single, const int* tile, const i64* nf);
 
@@ -200,8 +201,11 @@ int choose_method(int dim, int w, int requested, bool single, const int* tile, c
 void choose_tile(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
                  int method, int* tile);
 
-// Whether a 1D or 2D point set is ordered along strips (strip.cu): method 1 without an explicit
-// tile, where the strips' bins stay few enough to count.
+// Whether a requested tile is none, or that of the strips, as plans report it.
+bool strip_tile_or_none(int dim, int w, size_t complex_bytes, const int* requested);
+
+// Whether a 1D or 2D point set is ordered along strips (strip.cu): method 1 without a tile of
+// another shape, where the strips' bins stay few enough to count.
 bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* requested,
                 int method);
 

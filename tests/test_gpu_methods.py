@@ -267,3 +267,39 @@ def test_method4_rejected_outside_its_domain(cuda, engine):
     loc64 = [torch.zeros(4, device="cuda", dtype=torch.float64) for _ in range(3)]
     with pytest.raises(engine.InputError):
         engine.Plan(engine.Options(tol=1e-6, spread_method=4), -1, 4, loc64, [8, 8, 8])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", [4, 8, 9, 13])
+@pytest.mark.parametrize("modes", [[300], [40, 31], [20, 18, 16]])
+@pytest.mark.parametrize("type3", [False, True])
+def test_reported_method_and_tile_can_be_named(dtype, w, modes, type3, cuda, engine, oracle):
+    """A plan that names the method and tile that another reports is the same plan: same info (the
+    device memory, which differs between the kernels' point sets, included) and same result."""
+    torch = cuda
+    rng = np.random.default_rng(w)
+    rdt, cdt, npc = tdtypes(torch, dtype)
+    M = 2000
+    x = [torch.from_numpy(rng.uniform(-np.pi, np.pi, M)).to(rdt).cuda() for _ in modes]
+    c = torch.from_numpy((rng.standard_normal(M) + 1j * rng.standard_normal(M))).to(cdt).cuda()
+    infos, outs = [], []
+    for named in (False, True):
+        opt = engine.Options(tol=1e-5, n_spread=w)
+        if named:
+            opt.spread_method, opt.tile = infos[0]["spread_method"], tuple(infos[0]["tile"])
+        if type3:
+            plan = engine.PlanT3(opt, 1, M, x, M, x)
+            out = torch.empty(M, dtype=cdt, device="cuda")
+            plan.add_input(c, M)
+            plan.transform(out, M)
+        else:
+            plan = engine.Plan(opt, 1, M, x, modes)
+            out = torch.empty(int(np.prod(modes)), dtype=cdt, device="cuda")
+            plan.transform_type_1(c, out, col_strides(modes))
+        torch.cuda.synchronize()
+        infos.append(plan.info())
+        outs.append(out.cpu().numpy())
+        plan.close()
+    assert infos[0] == infos[1]
+    # the same kernels: sums in the order in which the points were sorted and the cells added to
+    assert oracle.rel_l2(outs[1], outs[0]) < (1e-6 if dtype == "float32" else 1e-14)
