@@ -7,8 +7,8 @@ synchronises and reports a recorded failure as NEONUFFT_INTERNAL_ERROR -- the co
 reference's debug-build sync-and-check after each launch (src/neonufft/gpu/util/runtime.hpp:27-30).
 
 The GPU test runs the small-case parity suites (the reference's type-1/2 and type-3 matrices,
-every spreading method and tile including the tensor-core spreading, the edge cases and the
-batches) and the large-set binning suite (whose records the checked build also checks for being
+every spreading method and tile including the tensor-core spreading, the strips, the wide 3D
+kernels, several vectors at once, the edge cases and the batches) and the large-set binning suite (whose records the checked build also checks for being
 a permutation of the points) in a child process that loads
 the checked library, so that any out-of-range index in those kernels fails the run.
 """
@@ -48,7 +48,8 @@ def test_parity_suites_under_the_checked_build(cuda):
         pytest.fail("the checked build is missing: python -m neonufft_b200.build --checked")
     suites = ["tests/test_gpu_type12.py", "tests/test_gpu_type3.py", "tests/test_gpu_methods.py",
               "tests/test_gpu_tcgen05.py", "tests/test_gpu_edges.py", "tests/test_gpu_batch.py",
-              "tests/test_gpu_binning.py"]
+              "tests/test_gpu_binning.py", "tests/test_gpu_strips.py",
+              "tests/test_gpu_zwin_wide.py", "tests/test_gpu_type1_many.py"]
     env = dict(os.environ, NEONUFFT_B200_LIB=str(CHECKED))
     res = subprocess.run([sys.executable, "-m", "pytest", "-m", "gpu", "-x", "-q",
                           "-p", "no:cacheprovider", *suites],

@@ -303,3 +303,66 @@ def test_reported_method_and_tile_can_be_named(dtype, w, modes, type3, cuda, eng
     assert infos[0] == infos[1]
     # the same kernels: sums in the order in which the points were sorted and the cells added to
     assert oracle.rel_l2(outs[1], outs[0]) < (1e-6 if dtype == "float32" else 1e-14)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("w", [2, 7, 12])
+@pytest.mark.parametrize("type_", [1, 2])
+@pytest.mark.parametrize("modes,tile", [([300], (512, 0, 0)), ([300], (37, 0, 0)),
+                                        ([61, 45], (64, 16, 0)), ([61, 45], (17, 9, 0)),
+                                        ([3, 2], (64, 16, 0))])
+def test_slabs_in_1d_and_2d(dtype, w, type_, modes, tile, cuda, engine, oracle):
+    """The shared-memory slabs of 1D and 2D plans that name a tile, against the strips of plans that
+    name none and the FP64 direct sums: tiles that do not divide the grid, and larger than it;
+    6000 points in one tile (several work items) beside scattered ones."""
+    rng = np.random.default_rng(w)
+    pts = [np.concatenate([0.3 + rng.uniform(0, 0.01, 6000), rng.uniform(-4, 4, 500)])
+           for _ in modes]
+    n_in = len(pts[0]) if type_ == 1 else int(np.prod(modes))
+    inp = rng.standard_normal(n_in) + 1j * rng.standard_normal(n_in)
+    slab, info = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w, tile=tile)
+    assert info["spread_method"] == 1
+    assert all(info["tile"][d] == min(tile[d], info["grid"][d]) for d in range(len(modes)))
+    strip, _ = run_t12(engine, cuda, dtype, 1, pts, inp, modes, type_, n_spread=w)
+    # the formula's kernel values in the slabs, the polynomials' in the strips: their difference on
+    # points that share their cells, 2.3 w 6e-8 a dimension (the square root rounded before it is
+    # multiplied by beta = 2.3 w), and sums of 6000 values in another order, u sqrt(6000 / 2) = 3e-6
+    same = 3e-6 + len(modes) * 2.3 * w * 6e-8
+    assert oracle.rel_l2(slab, strip) < (same if dtype == "float32" else 1e-13)
+    ref = direct(oracle, type_, 1, pts, inp, modes, dtype)
+    assert oracle.rel_l2(slab, ref) < width_bound(dtype, w)
+
+
+def test_grids_too_large_for_strips(cuda, engine, oracle):
+    """1D grids above 2^26 cells keep the slabs: a plan, and a type-3 plan whose sources lie on such
+    a grid (slabs) while its targets are sorted along strips with bins of 64 cells."""
+    torch = cuda
+    rng = np.random.default_rng(8)
+    M = 300
+    pts = rng.uniform(-np.pi, np.pi, M)
+    c = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    x, inp = torch.from_numpy(pts).cuda(), torch.from_numpy(c).cuda()
+    n = (1 << 25) + 5
+    plan = engine.Plan(engine.Options(tol=1e-9), 1, M, [x], [n])
+    assert plan.info()["grid"][0] > 1 << 26 and plan.info()["tile"][0] == 512
+    out = torch.empty(n, dtype=torch.complex128, device="cuda")
+    plan.transform_type_1(inp, out, [1])
+    modes = torch.from_numpy(rng.integers(-(n // 2), n // 2, 50)).cuda()
+    got = out[modes + n // 2].cpu().numpy()
+    plan.close()
+    del out
+    k = modes.cpu().numpy()
+    # phases up to 5e7 rad: 64-bit rounding of x leaves 1e-8
+    assert oracle.rel_l2(got, np.exp(1j * np.outer(k, pts)) @ c) < 1e-7
+
+    X, S = 7000.0, 8000.0
+    src, tgt = rng.uniform(-X, X, M), rng.uniform(-S, S, M)
+    plan = engine.PlanT3(engine.Options(tol=1e-9), 1, M, [torch.from_numpy(src).cuda()], M,
+                         [torch.from_numpy(tgt).cuda()])
+    assert plan.info()["spread_grid"][0] > 1 << 26 and plan.info()["tile"][0] == 512
+    out = torch.empty(M, dtype=torch.complex128, device="cuda")
+    plan.add_input(inp, M)
+    plan.transform(out, M)
+    torch.cuda.synchronize()
+    assert oracle.rel_l2(out.cpu().numpy(), np.exp(1j * np.outer(tgt, src)) @ c) < 1e-7
+    plan.close()
