@@ -1,5 +1,6 @@
 // Launchers of the z-window kernels (zwin.cuh) for kernel widths up to 8, the persistent kernels
 // over many transforms, and the spreading on tensor cores (method 4).
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -270,7 +271,13 @@ ZChunks make_chunks(i64 ncols, int nz, int w) {
   // overhead (w - 1 extra planes flushed, or RZ planes loaded, per chunk).
   const i64 target = 148 * 8 * 4;
   i64 count = (target + ncols - 1) / ncols;
-  const int min_len = 4 * w;
+  int min_len = 4 * w;
+  // A wide point takes a CTA long: on grids of few columns shorter chunks, until there are two for
+  // each SM (3e4 uniform points on 32^3 cells, w = 10, double precision: spreading 209 us with
+  // chunks of 4 w planes, 47 with 4; shared-memory slabs 173; interpolation 230, 52 and 121).
+  while (w > 8 && min_len > 4 && ncols * ((nz + min_len - 1) / min_len) < 2 * 148) {
+    min_len = std::max(4, min_len / 2);
+  }
   const i64 max_count = (nz + min_len - 1) / min_len;
   if (count > max_count) count = max_count;
   if (count < 1) count = 1;
