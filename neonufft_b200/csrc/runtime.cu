@@ -572,7 +572,7 @@ bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* 
 BinGeom widen_strips(const BinGeom& g, i64 M) {
   BinGeom wide = g;
   const int grow = g.dim - 1;  // 1D: more cells, 2D: more rows
-  const i64 limit = std::max(i64(1) << 16, 8 * M);
+  const i64 limit = std::max(i64(1) << 21, 8 * M);
   while (wide.total_tiles > limit && wide.tile[grow] < 64) {
     wide.tile[grow] *= 2;
     wide.ntiles[grow] = int((g.nf[grow] + wide.tile[grow] - 1) / wide.tile[grow]);

@@ -210,9 +210,11 @@ bool use_strips(int dim, int w, size_t complex_bytes, const i64* nf, const int* 
                 int method);
 
 // The bins of M strip-ordered points widened from one row (1D: cell) to as many as 64, until they
-// number no more than eight to a point: 8 bytes of counts and offsets each, cleared and scanned
-// with every new point set (set_points of 1e3 points on 6.7e7 cells in 1D: 464 us and 537 MB with
-// bins of a cell, 55 us and 8 MB; on 16000^2 cells in 2D 251 and 55 us, 256 and 4 MB).
+// number no more than eight to a point, or 2^21: 8 bytes of counts and offsets each, cleared and
+// scanned with every new point set (set_points of 1e3 points on 6.7e7 cells in 1D: 464 us and 537 MB
+// with bins of a cell, 62 us and 17 MB; on 16000^2 cells in 2D 251 us and 256 MB, 62 us and 16 MB).
+// Fewer bins would save less than a set costs that turns out to be crowded and is binned again (3e4
+// clustered points on 3000 x 2800 cells: 47 us, 100 us if their 1e6 bins were widened first).
 BinGeom widen_strips(const BinGeom& g, i64 M);
 
 // Tile of a strip-ordered point set: bins of one row (spreading walks the points row by row), or
