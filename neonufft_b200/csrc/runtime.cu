@@ -352,7 +352,9 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
     if (bin(wide, x, M, stream, u32(kCrowdedSparse * rows)) <= kWorkItemPoints) return;
   }
   const bool sparse = strip_sparse(g, M);
-  const u32 crowded = bin(g, x, M, stream, sparse ? kCrowdedSparse : kCrowdedDense);
+  // (the runs of 2^21 dense points or fewer are shorter than crowded ones may be)
+  const u32 dense_least = M > (i64(1) << 21) ? kCrowdedDense : 0;
+  const u32 crowded = bin(g, x, M, stream, sparse ? kCrowdedSparse : dense_least);
   if (crowded <= kWorkItemPoints) return;
   if (sparse) {
     crowded_.reserve(size_t((M + kStripUnit - 1) / kStripUnit));
