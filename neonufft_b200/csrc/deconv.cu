@@ -201,6 +201,7 @@ void launch_downsample(const DeconvArgs<T>& a, const cplx_t<T>* fine, cplx_t<T>*
                        cudaStream_t stream) {
   const i64 m1 = a.dim > 1 ? a.modes[1] : 1;
   const i64 m2 = a.dim > 2 ? a.modes[2] : 1;
+  // (the public limits of the interface; the launch itself has none)
   if (m1 > 65535 || m2 > 65535) throw_input("mode count above 65535 in dimension 1 or 2");
   const RowTasks t = row_tasks(a.modes[0], m1, m2);
   downsample_kernel<T><<<deconv_grid(t), kDeconvThreads, 0, stream>>>(a, t, fine, out);
@@ -212,6 +213,7 @@ void launch_upsample(const DeconvArgs<T>& a, const cplx_t<T>* in, cplx_t<T>* fin
                      cudaStream_t stream) {
   const i64 n1 = a.dim > 1 ? a.nf[1] : 1;
   const i64 n2 = a.dim > 2 ? a.nf[2] : 1;
+  // (the public limits of the interface; the launch itself has none)
   if (n1 > 65535 || n2 > 65535) throw_input("fine grid above 65535 in dimension 1 or 2");
   const RowTasks t = row_tasks(a.nf[0], n1, n2);
   const bool vec = a.nf[0] % 2 == 0 && reinterpret_cast<uintptr_t>(fine) % 16 == 0;

@@ -12,8 +12,9 @@ namespace nnb {
 
 template <typename T>
 struct EsPoly {
-  // degree 9 in single, 16 in double precision: the fits are off by about 1e-9 and 1e-16 of the
-  // kernel's peak, below the rounding of the direct formula
+  // degree 9 in single, 16 in double precision: below the rounding of the direct formula where they
+  // are used (es_poly in params.hpp; at w = 8 and upsampling 2 the inner pieces are off by 1e-10
+  // and up to 8e-16 of the kernel's peak, the edge piece by 1.6e-8 in single precision)
   static constexpr int NE = sizeof(T) == 4 ? 5 : 9;
   static constexpr int NO = sizeof(T) == 4 ? 5 : 8;
   T e[8][NE];  // coefficients of t^0, t^2, ... of piece k

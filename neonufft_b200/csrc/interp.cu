@@ -5,8 +5,9 @@
 // order.
 //
 // Method 1 in 3D, or with an explicit tile (1D and 2D otherwise: strip.cu): a CTA of up to 4 warps
-// covers as many consecutive tiles (bins) along the last dimension and stages their union plus the (w-1)-cell halo into shared memory once
-// (coalesced along x, periodic wrap, padded strides, tile_layout.cuh). Each warp walks one
+// covers as many consecutive tiles (bins) along the last dimension and stages their union plus the
+// (w-1)-cell halo into shared memory once (coalesced along x, periodic wrap, padded strides,
+// tile_layout.cuh). Each warp walks one
 // tile's bin-sorted points in batches of 32 (lane j loads point j's record and evaluates its
 // w*d kernel values, all in parallel); then, one point at a time, lane r contracts footprint
 // row r (3D: (dy, dz); 2D: cell (dx, dy)) against kx, and a shuffle reduction forms the

@@ -92,7 +92,9 @@ struct SpreadArgs {
   T beta;
   T c;
   EsPoly<T> es;
-  int method;  // 1: warp-private slabs, 2: thread per point, 3: z-window, 4: z-window on tensor cores (zwin.cu)
+  // 1: strips if g.strip, else warp-private slabs; 2: thread per point; 3: z-window; 4: z-window on
+  // tensor cores (zwin.cu); 5: tcgen05 tensor cores (spread_tc.cu)
+  int method;
 };
 template <typename T>
 void launch_spread(const SpreadArgs<T>& a, cudaStream_t stream);
@@ -129,7 +131,7 @@ struct InterpArgs {
   T beta;
   T c;
   EsPoly<T> es;
-  int method;  // 1: warp per point, 2: thread per point, 3: z-window (zwin.cu)
+  int method;  // 1: strips if g.strip, else warp per point; 2: thread per point; 3 to 5: z-window
 };
 template <typename T>
 void launch_interp(const InterpArgs<T>& a, cudaStream_t stream);

@@ -65,8 +65,9 @@ PhiHatQuad phi_hat_quadrature(const KernelParam& kp);
 // ES kernel value in double precision (with the plan's rounded beta and c).
 double es_kernel(const KernelParam& kp, double x);
 
-// Polynomials of the kernel's pieces, and which of them are accurate enough to be used: within
-// 3e-8 (T = float) or 2e-16 (double) of the kernel's peak, else that piece stays with the formula.
+// Polynomials of the kernel's pieces, and where they are accurate enough to be used (errors relative
+// to the kernel's peak): the two edge pieces stay with the formula unless theirs are within 3e-8
+// (T = float) or 2e-16 (double), and all pieces do unless the inner ones are within 3e-8 or 1e-15.
 template <typename T>
 EsPoly<T> es_poly(const KernelParam& kp);
 

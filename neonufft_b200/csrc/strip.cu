@@ -20,6 +20,10 @@
 // staged in shared memory by one lane each: kx placed over the strip's cells and ky over the
 // window, zero elsewhere, so that the register indices are fixed.
 //
+// 2D points that are sparse on average are added to the grid directly, but for the places where
+// they crowd (spread_sparse_unit, spread_mixed_kernel). Bins may hold several cells (1D) or rows of a
+// strip (2D, direct spreading and interpolation only) where rows would outnumber the points by far.
+//
 // Interpolation: one thread per point reads its W^d cells through the L1. Neighbouring threads
 // hold neighbouring points, so a warp's load of one (dx, dy) falls on a few rows of one strip.
 //

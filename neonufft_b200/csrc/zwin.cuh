@@ -1,33 +1,34 @@
 // 3D ES spreading and interpolation with a sliding z-window held in registers (method 3).
 //
-// Replaces, for 3D plans with kernel width w <= 8, the reference's spreading
+// Replaces, for 3D plans, the reference's spreading
 // (src/neonufft/gpu/kernels/spreading_kernel.cu:477-715, one global float atomic per cell and
 // point) and interpolation (src/neonufft/gpu/kernels/interpolation_kernel.cu, one thread per
 // point reading w^3 cells from global memory).
 //
-// Points are binned by (x tile of TX cells, y tile of 8 cells, single z plane), and the bins of
+// Points are binned by (x tile of TX cells, y tile of TY cells, single z plane), and the bins of
 // one (x, y) column are consecutive in plane order (BinGeom::zmajor), so the points of a column
 // and range of planes are one contiguous run of records. One CTA walks one column over a chunk
-// of planes. Its region is P0 x P1 cells in (x, y), P0 = TX + w - 1 and P1 = 8 + w - 1 <= 15,
-// times a window of RZ >= w consecutive planes [t, t + RZ):
+// of planes. Its region is P0 x P1 cells in (x, y), P0 = TX + w - 1 and P1 = TY + w - 1, times a
+// window of RZ >= w consecutive planes [t, t + RZ): 4 or 8 planes up to w = 8, exactly w above.
 //  * thread (a, b) keeps in registers the whole region row y = a (P0 cells, as pairs of
-//    neighbouring cells) of the window plane p = b (mod RZ). The 16 rows are split over the
-//    warps, LA = 32 / RZ rows per warp, so for a point whose footprint covers rows
+//    neighbouring cells) of the window plane p = b (mod RZ), or of two planes, RZ / 2 apart
+//    (ZShape::PZ). The RY >= P1 rows are split over the warps, LA rows per warp (as many as its
+//    32 lanes hold with RZ / PZ lanes each), so for a point whose footprint covers rows
 //    [ly, ly + w) a warp either owns some of them or skips the point with a warp-uniform
 //    branch; no thread holds a cell that another thread updates, so there are no atomics and
 //    no shared-memory traffic per cell;
-//  * the run of points is staged in shared memory 64 at a time (double-buffered, one barrier
-//    per batch, spread over all warps): kx over the region's x range, ky over the 16 rows and
-//    kz over the RZ planes, each zero outside the footprint, so that every thread applies
-//    them with fixed register indices and no range tests;
+//  * the run of points is staged in shared memory 32 to 64 at a time (ZShape::BATCH;
+//    double-buffered, one barrier per batch, spread over all warps): kx over the region's x
+//    range, ky over the rows and kz over the RZ planes, each zero outside the footprint, so that
+//    every thread applies them with fixed register indices and no range tests;
 //  * each owning thread updates its row with packed two-float FMAs (fma.rn.f32x2 on sm_100a),
 //    one for the real and one for the imaginary parts of two neighbouring cells;
 //  * when the next point starts on a later plane, the window advances: spreading adds each
 //    completed plane to the fine grid (float2 / double2 atomics: neighbouring columns and
 //    chunks overlap by the halo); interpolation reloads the threads that held it with the
 //    plane RZ further on (plain loads: a cp.async prefetch one plane ahead measured no faster);
-//  * interpolation reduces the row sums of eight points at a time through a per-warp
-//    shared-memory transpose, then over warps.
+//  * interpolation reduces the row sums of eight points at a time (four of wide kernels) through
+//    a per-warp shared-memory transpose, then over warps.
 #pragma once
 
 #include <type_traits>
@@ -144,7 +145,8 @@ template <typename T, int W, int TX, bool SPREAD, int TY = 8, int PZ = 1, bool P
 __device__ __forceinline__ void stage_warp(ZSlot<T, W, TX, TY, PZ>* slots, const PointRec<T>* recs,
                                            int count, const cplx_t<T>* in,
                                            const cplx_t<T>* prephase,
-                                           const EsPoly<T>& es, T beta, T c, int lane, i64 num, const cplx_t<T>* in2 = nullptr,
+                                           const EsPoly<T>& es, T beta, T c, int lane, i64 num,
+                                           const cplx_t<T>* in2 = nullptr,
                                            cplx_t<T>* v2_out = nullptr) {
   using S = ZShape<T, W, TX, TY, PZ>;
   using C = cplx_t<T>;
