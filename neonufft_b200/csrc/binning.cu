@@ -78,7 +78,7 @@ __device__ __forceinline__ i64 tile_linear_d(const BinGeom& g, const i64 (&t)[3]
 
 // Where the count of bin b lies: eight bins in a row go to eight runs of n8 counts. Atomics on
 // one 32-byte sector of the L2 wait for one another, and clustered points hit neighbouring bins
-// (3e6 points of a Gaussian cluster on 192^3 cells: 303 -> 156 us); the scan reads the eight runs side by
+// (3e6 points of a Gaussian cluster on 192^3 cells: 303 -> 163 us); the scan reads the eight runs side by
 // side, each coalesced.
 __host__ __device__ __forceinline__ i64 count_slot(i64 b, i64 n8) { return (b & 7) * n8 + (b >> 3); }
 

@@ -80,7 +80,7 @@ struct ZShape {
   static constexpr int SPREAD_CTAS = 65536 / (NT * 92);
   // The wide kernels have a budget of 112 registers (3 CTAs of 192 threads at w = 10 in double
   // precision, a few spills; uncapped, ptxas takes 157 and 2 CTAs fit: spreading 5e5 points
-  // 512 -> 475 us, interpolation 628 -> 568 us).
+  // 512 -> 453 us, interpolation 628 -> 567 us).
   static constexpr int WIDE_CTAS = 65536 / (NT * 112) > 0 ? 65536 / (NT * 112) : 1;
   static constexpr int INTERP_CTAS =
       WIDE ? WIDE_CTAS : (PZ > 1 ? PZ_INTERP_CTAS : (sizeof(T) == 4 ? 6 : 5));

@@ -3,7 +3,7 @@
 //
 // The shared-memory slabs that took these widths (spread.cu, interp.cu) are bound by the chain of
 // shared-memory accesses from point to point: 5e5 points on 128 x 120 x 128 cells, w = 10, double
-// precision, spread in 2.87 ms and interpolated in 1.56 ms; here 0.47 and 0.57 ms, bound by the
+// precision, spread in 2.87 ms and interpolated in 1.56 ms; here 0.45 and 0.57 ms, bound by the
 // FP64 pipe and, at a quarter of a point per cell, by the latency of the planes that enter and
 // leave the window.
 #include "kernels.cuh"
