@@ -367,7 +367,7 @@ void PointSet<T>::build(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t st
 template <typename T>
 u32 PointSet<T>::bin(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t stream, u32 crowded) {
   g_ = g;
-  M_ = M;
+  M_ = 0;  // no points, should an array below not be had
   const i64 nt = g.total_tiles;
   const i64 nc = 8 * count_run(nt);
   // behind the counts the error flag and the points of crowded bins: one memset for all
@@ -382,6 +382,7 @@ u32 PointSet<T>::bin(const BinGeom& g, CoordPtrs<T> x, i64 M, cudaStream_t strea
     work_start_.reserve(size_t(nt + 1));
     work_owner_.reserve(size_t(nt + M / kWorkItemPoints + 2));
   }
+  M_ = M;
   NNB_CUDA(cudaMemsetAsync(counts_.data(), 0, sizeof(u32) * (nc + 2), stream));
   int* err = reinterpret_cast<int*>(counts_.data() + nc);
   launch_bin_count<T>(g, x, M, counts_.data(), ranks_.data(), err, stream);

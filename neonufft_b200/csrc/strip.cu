@@ -538,8 +538,8 @@ void launch_spread_strip_w(const SpreadArgs<T>& a, cudaStream_t stream) {
       dim3 grid{unsigned(ctas), unsigned(a.batch), 1u};
       // The crowded units go to windows: added directly, the points of a cluster queue up for a
       // few sectors, and a cell's sum is rounded once per point (1.2e6 points of one sign, sigma
-      // 0.01 rad, 3000^2 cells, w = 7: 1669 us and a relative error of 2e-4 against 78 us and
-      // 9e-7).
+      // 0.01 rad, 3000^2 cells, w = 7: 1669 us and a relative error of 2e-4 against 66 us and
+      // 5e-7).
       if (a.pts.crowded_points == 0) {
         spread_sparse_kernel<T, W><<<grid, 32 * kStripWarps, 0, stream>>>(a, aligned);
       } else {

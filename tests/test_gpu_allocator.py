@@ -82,3 +82,45 @@ def test_plan_on_a_16_byte_aligned_allocator(dtype, cuda, engine, oracle):
     sample = rng.integers(0, M, 400)
     ref2 = direct(oracle, 2, -1, [p[sample] for p in pts], f, modes, dtype)
     assert oracle.rel_l2(two[sample], ref2) < bound
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_failed_set_points_leaves_no_points(dim, cuda, engine):
+    """A set_points whose arrays cannot be had raises MemoryAllocError and leaves the plan without
+    points, not with the new number of points and missing records; the next one works."""
+    torch = cuda
+
+    class Limited(OffsetAllocator):
+        limit = 1 << 40
+
+        def allocate(self, size):
+            if size > self.limit:
+                return 0
+            return super().allocate(size)
+
+    alloc = Limited(torch)
+    modes = [12] * dim
+    nm = int(np.prod(modes))
+
+    def points(M):
+        return [torch.rand(M, device="cuda") * 6 - 3 for _ in range(dim)]
+
+    few, many = points(100), points(200_000)
+    c = torch.ones(200_000, dtype=torch.complex64, device="cuda")
+    plan = engine.Plan(engine.Options(tol=1e-5), -1, 100, few, modes, device_alloc=alloc)
+    alloc.limit = 1 << 20  # the records of 200 000 points take 6.4 MB
+    with pytest.raises(engine.MemoryAllocError):
+        plan.set_points(200_000, many)
+    assert plan.info()["num_in"] == 0
+    out = torch.ones(nm, dtype=torch.complex64, device="cuda")
+    plan.transform_type_1(c, out, col_strides(modes))
+    torch.cuda.synchronize()
+    assert float(out.abs().max()) == 0.0
+    alloc.limit = 1 << 40
+    plan.set_points(200_000, many)
+    plan.transform_type_1(c, out, col_strides(modes))
+    torch.cuda.synchronize()
+    # the mode 0 of ones is their number (CMCL order: mode 0 in the middle)
+    centre = sum(m // 2 * s for m, s in zip(modes, col_strides(modes)))
+    assert abs(complex(out[centre].item()) - 200_000) < 1e-3 * 200_000
+    plan.close()
